@@ -1060,7 +1060,7 @@ int agpu_create(const agpu_params* params, agpu_handle** out) {
     }
   }
   if (!rc) {
-    h->tg = make_tiles(g, p.nx, p.ny, p.nz);
+    h->tg = make_tiles(g, p.nx, p.ny, p.nz, h->fp32);
     for (int ic = 0; ic < p.nsp_run && !rc; ++ic) {
       rc |= dmalloc((void**)&h->key[ic], sizeof(int) * capmax);
       rc |= dmalloc((void**)&h->perm[ic], sizeof(int) * capmax);

@@ -11,6 +11,9 @@ namespace agpu {
 // kernel gives each warp one x-row of a tile, one node per lane, so that its
 // shared-memory stencil reads are 32 consecutive words.
 constexpr int TILE3_X = 32, TILE3_Y = 4, TILE3_Z = 4;
+// The FP64 form's 3D tile is half as deep: its fields and two groups of
+// deposit data of eight rows fit an SM's shared memory twice.
+constexpr int TILE64_Y = 4, TILE64_Z = 2;
 constexpr int TILE2_X = 32, TILE2_Y = 8;
 
 struct TileArgs32 {
@@ -53,7 +56,7 @@ struct TileArgs64 {
   unsigned int* err;
 };
 
-TileGeo make_tiles(const Geo& g, int nx, int ny, int nz);
+TileGeo make_tiles(const Geo& g, int nx, int ny, int nz, bool fp32);
 int tile_push32(const TileArgs32& a, cudaStream_t st, int sms);
 int tile32_list_cap(int ndim);
 // the cubic shape extension (agpu_tile32c.cu)
