@@ -38,6 +38,7 @@ UNITS = [
     ("agpu_noalloc.cu", ["-fmad=false"]),
     ("agpu_envar.cu", ["-fmad=false"]),
     ("agpu_env.cu", ["-fmad=false"]),
+    ("agpu_env_tile.cu", ["-fmad=false"]),
     ("agpu_beam.cu", ["-fmad=false"]),
     ("agpu_ionz.cpp", []),
     ("agpu_batch.cpp", ["-Xcompiler", "-pthread"]),

@@ -536,6 +536,54 @@ int reorder_records(agpu_handle* h, int ic) {
   return 0;
 }
 
+// Arguments of the FP64 tile kernels for species ic.
+void tile_args64(const agpu_handle* h, int ic, int initial_time, TileArgs64& a) {
+  const agpu_params& p = h->p;
+  a.g = h->g;
+  a.t = h->tg;
+  a.ebf = h->ebf;
+  a.jc = h->jc;
+  double* b = h->part[ic];
+  long long cp = h->cap[ic];
+  a.x = b;
+  a.y = b + cp;
+  if (p.ndim == 3) {
+    a.z = b + 2 * cp;
+    a.px = b + 3 * cp;
+    a.py = b + 4 * cp;
+    a.pz = b + 5 * cp;
+    a.slot = b + 6 * cp;
+  } else {
+    a.z = nullptr;
+    a.px = b + 2 * cp;
+    a.py = b + 3 * cp;
+    a.pz = nullptr;
+    a.slot = b + 4 * cp;
+  }
+  a.perm = h->perm[ic];
+  a.tstart = h->tstart[ic];
+  a.key = h->key[ic];
+  a.hist = h->hist[ic];
+  a.xmn = p.xmn;
+  a.ymn = p.ymn;
+  a.zmn = p.zmn;
+  a.dx_inv = p.dx_inv;
+  a.dy_inv = p.dy_inv;
+  a.dz_inv = p.dz_inv;
+  a.dt = p.dt;
+  a.dth = 0.5 * p.dt;
+  a.lfact = p.lorentz_fact[ic];
+  a.gxmin = p.gxmin;
+  a.gxmax = p.gxmax;
+  a.gymin = p.gymin;
+  a.gymax = p.gymax;
+  a.gzmin = p.gzmin;
+  a.gzmax = p.gzmax;
+  a.vdt = comoving_vdt(p);
+  a.initial = initial_time ? 1 : 0;
+  a.err = &h->d_cnt->err;
+}
+
 // Tiled gather + push + deposit of species ic, then the next binning from
 // the keys the kernel wrote.  Removed particles stay stored (key nkeys)
 // until the next compaction.
@@ -579,49 +627,7 @@ int tiled_push(agpu_handle* h, int ic, int initial_time, agpu_step_out* out) {
       h->timers.launches_total += tile_push32(a, h->st, h->sms) - 1;
   } else {
     TileArgs64 a;
-    a.g = h->g;
-    a.t = h->tg;
-    a.ebf = h->ebf;
-    a.jc = h->jc;
-    double* b = h->part[ic];
-    long long cp = h->cap[ic];
-    a.x = b;
-    a.y = b + cp;
-    if (p.ndim == 3) {
-      a.z = b + 2 * cp;
-      a.px = b + 3 * cp;
-      a.py = b + 4 * cp;
-      a.pz = b + 5 * cp;
-      a.slot = b + 6 * cp;
-    } else {
-      a.z = nullptr;
-      a.px = b + 2 * cp;
-      a.py = b + 3 * cp;
-      a.pz = nullptr;
-      a.slot = b + 4 * cp;
-    }
-    a.perm = h->perm[ic];
-    a.tstart = h->tstart[ic];
-    a.key = h->key[ic];
-    a.hist = h->hist[ic];
-    a.xmn = p.xmn;
-    a.ymn = p.ymn;
-    a.zmn = p.zmn;
-    a.dx_inv = p.dx_inv;
-    a.dy_inv = p.dy_inv;
-    a.dz_inv = p.dz_inv;
-    a.dt = p.dt;
-    a.dth = 0.5 * p.dt;
-    a.lfact = p.lorentz_fact[ic];
-    a.gxmin = p.gxmin;
-    a.gxmax = p.gxmax;
-    a.gymin = p.gymin;
-    a.gymax = p.gymax;
-    a.gzmin = p.gzmin;
-    a.gzmax = p.gzmax;
-    a.vdt = comoving_vdt(p);
-    a.initial = initial_time ? 1 : 0;
-    a.err = &h->d_cnt->err;
+    tile_args64(h, ic, initial_time, a);
     tile_push64(a, h->st);
   }
   CK(cudaGetLastError());
@@ -665,7 +671,7 @@ __global__ void k_shift_cells(int* cell, float* ox, long long n, int nshx, int n
 }
 
 // lp_window_xshift (src/dynamics/window.f90:276-347).
-int window_xshift(agpu_handle* h, int witr, int init_iter, agpu_step_out* out) {
+int window_xshift(agpu_handle* h, int witr, int init_iter, agpu_step_out* out, bool alive) {
   agpu_params& p = h->p;
   if (init_iter == 0) {
     h->xlapse = 0.0;
@@ -703,7 +709,7 @@ int window_xshift(agpu_handle* h, int witr, int init_iter, agpu_step_out* out) {
       CK(cudaGetLastError());
       h->timers.launches_total += 1;
     }
-    long long before = h->np[ic];
+    const long long before = alive && h->binned[ic] ? h->nalive[ic] : h->np[ic];
     int rc = compact_species(h, ic, true);
     if (rc) return rc;
     out->removed[ic] += before - h->np[ic];
@@ -731,7 +737,7 @@ int window_xshift(agpu_handle* h, int witr, int init_iter, agpu_step_out* out) {
 // so every lattice column not yet injected) moves by -vb w_nst dt, the
 // particles at or left of gxmin (or past gxmax) are dropped along x only and
 // the columns that entered the box are injected.
-int comoving_coordinate(agpu_handle* h, double vb, int w_nst, int loc_it, agpu_step_out* out) {
+int comoving_coordinate(agpu_handle* h, double vb, int w_nst, int loc_it, agpu_step_out* out, bool alive) {
   agpu_params& p = h->p;
   if (loc_it == 0) return 0;
   const double dt_step = p.dt;
@@ -744,7 +750,7 @@ int comoving_coordinate(agpu_handle* h, double vb, int w_nst, int loc_it, agpu_s
   }
   for (int ic = 0; ic < p.nsp; ++ic) {
     if (h->np[ic] <= 0) continue;
-    long long before = h->np[ic];
+    const long long before = alive && h->binned[ic] ? h->nalive[ic] : h->np[ic];
     int rc = compact_species(h, ic, true);
     if (rc) return rc;
     out->removed[ic] += before - h->np[ic];
@@ -774,18 +780,19 @@ long long xadv_launches(const agpu_handle* h) { return h->xadv.tmp ? 6 + 2LL * h
 
 // lp_run (src/dynamics/pic_evolve_in_time.f90 callers): the moving window
 // (w_speed > 0) or the comoving frame's coordinate step (w_speed < 0), every
-// w_sh steps inside [wi_time, wf_time)
-int window_or_comoving(agpu_handle* h, int iter, double t, agpu_step_out* out) {
+// w_sh steps inside [wi_time, wf_time); alive: records dropped in earlier
+// steps and still stored were counted then and are not counted as removed here
+int window_or_comoving(agpu_handle* h, int iter, double t, agpu_step_out* out, bool alive = false) {
   const agpu_params& p = h->p;
   if (p.w_sh <= 0 || !(t >= p.wi_time && t < p.wf_time) || iter % p.w_sh != 0) return 0;
   int rc = 0;
   if (p.w_speed > 0.0) {
     ph_begin(h, PH_WINDOW);
-    rc = window_xshift(h, p.w_sh, iter, out);
+    rc = window_xshift(h, p.w_sh, iter, out, alive);
     ph_end(h, PH_WINDOW);
   } else if (p.w_speed < 0.0) {
     ph_begin(h, PH_WINDOW);
-    rc = comoving_coordinate(h, -p.w_speed, p.w_sh, iter, out);
+    rc = comoving_coordinate(h, -p.w_speed, p.w_sh, iter, out, alive);
     ph_end(h, PH_WINDOW);
   }
   return rc;
@@ -2225,20 +2232,29 @@ int agpu_env_run(agpu_handle* h, int32_t iter, double t, agpu_step_out* out) {
   agpu_params& p = h->p;
   const Geo& g = h->g;
   const int ic = 0;
-  if (int rc = drop_removed(h, ic)) return rc;
+  // The particle steps run on tiles, except in the deterministic mode, whose
+  // serial sums follow the particle order, and for the iform = 2 deposit.
+  const bool tiles = !h->deterministic && h->key[ic] && p.iform < 2 && h->np[ic] > 0;
+  if (int rc = tiles ? refresh_counts(h) : drop_removed(h, ic)) return rc;
   CK(cudaMemsetAsync(h->d_cnt, 0, sizeof(Counters), h->st));
   // Every `every` calls the records move in memory along the tile
   // permutation (tile, row inside the tile, offset octant): a warp then
-  // covers consecutive x cells of one tile row, so its stencil loads share
-  // cache lines and its FP64 atomics mostly hit different addresses.  Not in
-  // the deterministic mode, whose serial sums follow the particle order.
+  // covers consecutive x cells of one tile row, so its record loads (and the
+  // per-particle kernels' stencils) share cache lines.
   const int every = h->sort_interval > 0 ? h->sort_interval : 8;
-  if (!h->deterministic && h->key[ic] && h->np[ic] > 0 && h->env_steps % every == 0) {
+  if (!h->deterministic && h->key[ic] && h->np[ic] > 0) {
     ph_begin(h, PH_SORT);
-    if (int rc = rebin(h, ic)) return rc;
-    if (int rc = reorder_records(h, ic)) return rc;
+    if (h->env_steps % every == 0) {
+      if (!h->binned[ic] || !tiles)
+        if (int rc = rebin(h, ic)) return rc;
+      if (int rc = reorder_records(h, ic)) return rc;
+    }
+    if (tiles && !h->binned[ic])
+      if (int rc = rebin(h, ic)) return rc;
     ph_end(h, PH_SORT);
   }
+  if (int rc = refresh_counts(h)) return rc;  // deferred counts: the binning's alive count
+  if (!tiles) h->binned[ic] = false;          // the particles move without new keys
   h->env_steps++;
   EnvArgs a;
   a.g = g;
@@ -2298,30 +2314,55 @@ int agpu_env_run(agpu_handle* h, int32_t iter, double t, agpu_step_out* out) {
   // jc(:,:,:,:) = 0; env_amp_prepare
   CK(cudaMemsetAsync(h->env_av, 0, sizeof(double) * c3 * (g.ndim + 1), h->st));
   env_amp_grad(a, h->st, h->sms);
+  EnvTileArgs ta;
+  const long long alive0 = h->nalive[ic];
+  if (tiles) {
+    tile_args64(h, ic, 0, ta);
+    ta.av = h->env_av;
+    ta.den = h->env_den;
+    hist_reset(h->hist[ic], h->tstart[ic], h->tg, h->np[ic], false, nullptr, h->st);
+  }
   // set_env_acc, lpf_env_momenta, set_env_density (jc(:,:,:,1) = 0 first)
   CK(cudaMemsetAsync(h->env_den, 0, sizeof(double) * c3, h->st));
-  env_acc_momenta(a, h->st, h->sms, h->deterministic);
+  if (tiles) env_acc_tile(ta, h->st);
+  else env_acc_momenta(a, h->st, h->sms, h->deterministic);
   // env_den_collect; jc(3) = jc(1)
   env_den_collect(a, h->st, h->sms);
   // advance_lpf_envelope, env_fields_average
   env_advance(a, h->st, h->sms);
   // set_env_grad_interp, lpf_env_positions, cell_part_dist, curr_accumulate
   CK(cudaMemsetAsync(h->jc, 0, sizeof(double) * c3 * g.nc, h->st));
-  env_positions_deposit(a, h->st, h->sms, h->deterministic);
+  if (tiles) env_pos_tile(ta, h->st);
+  else env_positions_deposit(a, h->st, h->sms, h->deterministic);
   CK(cudaGetLastError());
   ph_end(h, PH_PUSH);
   h->timers.launches_push_deposit += 2;
   h->timers.launches_total += 12 + (g.ndim == 3 ? 2 : 0) + (a.vdt > 0. ? 1 : 0);
-  h->timers.pushes += a.np;
-  if (int rc = read_counters(h)) return rc;
+  h->timers.pushes += tiles ? alive0 : a.np;
   int rc = 0;
-  if (h->h_cnt->removed > 0) {
+  if (tiles) {
+    // the next binning from the keys of the position step; removed records
+    // stay stored (key nkeys) until the next compaction
     ph_begin(h, PH_SORT);
-    const long long before = h->np[ic];
-    rc = compact_species(h, ic, false);
+    const int nl = bin_finish(h->key[ic], h->np[ic], h->tg, h->hist[ic], h->tstart[ic], h->cursor, h->perm[ic],
+                              h->scan_tmp, h->st, h->sms);
+    CK(cudaGetLastError());
+    h->timers.launches_total += 1 + nl;  // histogram reset, scan and scatter
+    CK(cudaMemcpyAsync(&h->d_cnt->alive, h->tstart[ic] + h->tg.nkeys, sizeof(int), cudaMemcpyDeviceToDevice, h->st));
+    if ((rc = read_counters(h))) return rc;
     ph_end(h, PH_SORT);
-    if (rc) return rc;
-    out->removed[ic] += before - h->np[ic];
+    h->nalive[ic] = h->h_cnt->alive;
+    out->removed[ic] += alive0 - h->nalive[ic];
+  } else {
+    if ((rc = read_counters(h))) return rc;
+    if (h->h_cnt->removed > 0) {
+      ph_begin(h, PH_SORT);
+      const long long before = h->np[ic];
+      rc = compact_species(h, ic, false);
+      ph_end(h, PH_SORT);
+      if (rc) return rc;
+      out->removed[ic] += before - h->np[ic];
+    }
   }
   // curr_mpi_collect (djc folded into the E update), advance_lpf_fields
   ph_begin(h, PH_YEE);
@@ -2333,7 +2374,7 @@ int agpu_env_run(agpu_handle* h, int32_t iter, double t, agpu_step_out* out) {
   h->timers.launches_yee += 1;
   h->timers.launches_total += ((p.ndim == 3) ? 3 : 2) + 6 + xadv_launches(h);
   h->timers.yee_cells += (long long)p.nx * p.ny * (p.ndim == 3 ? p.nz : 1);
-  if ((rc = window_or_comoving(h, iter, t, out))) return rc;
+  if ((rc = window_or_comoving(h, iter, t, out, true))) return rc;
   if (int rc_ = read_counters(h)) return rc_;
   for (int q = 0; q < 4; ++q) out->np[q] = h->binned[q] ? h->nalive[q] : h->np[q];
   out->xmn = p.xmn;

@@ -10,8 +10,9 @@
 // inputs the grid arrays and particles equal the CPU restatement bit for bit
 // (the density and current sums in the deterministic, serial mode).  Grid
 // kernels run one thread per node; the particle kernels one thread per
-// particle with global-memory stencils (the envelope route runs on the PWFA
-// set-up, not on the tiled benchmark path).  The stretch factors
+// particle with global-memory stencils: they serve the deterministic mode
+// (one thread) and the iform = 2 deposit, the rest runs on tiles
+// (agpu_env_tile.cu).  The stretch factors
 // loc_yg/loc_zg(:,3:4) of a uniform grid are 1 and are left out (x * 1 == x
 // exactly).
 #include "agpu_env.h"
@@ -85,102 +86,6 @@ __global__ void k_env_grad(double* av, Geo g, double dxi, double dyi, double dzi
 }
 
 __device__ __forceinline__ bool in_stencil(int lo, int n) { return lo >= 1 && lo + 2 <= n; }
-
-// The atomic-mode Esirkepov deposit of one 3D move: the terms of
-// esirkepov3d (grid_part_connect.f90:1168-1334) with every window loop
-// unrolled over its five slots, so the window arrays stay in registers, and
-// where the old-plane and new-plane terms of a component land on the same
-// node (the particle keeps its z node for Jx and Jy, its y node for Jz) the
-// two terms are summed before one atomic add instead of two.  The sums then
-// round differently from the reference's two adds (the serial mode keeps
-// esirkepov3d); the atomic mode's sum order is not the reference's anyway.
-__device__ __forceinline__ bool esirkepov3d_sum(const Geo& g, double* jc, const double xn[3], const double xo[3],
-                                                float wght) {
-  double ax0[3], ay0[3], az0[3], ax1[3], ay1[3], az1[3];
-  double axh[5], ayh[5], azh[5], axh0[5], axh1[5], ayh0[5], ayh1[5];
-  double currx[5], curry[5], currz[5];
-  const int ii0 = qden64(xo[0], ax0), jj0 = qden64(xo[1], ay0), kk0 = qden64(xo[2], az0);
-  const int i = qden64(xn[0], ax1), j = qden64(xn[1], ay1), k = qden64(xn[2], az1);
-  if ((unsigned)(i - ii0 + 1) > 2u || (unsigned)(j - jj0 + 1) > 2u || (unsigned)(k - kk0 + 1) > 2u) return false;
-  const double w = (double)wght;
-  const int ih = i - ii0 + 1, jh = j - jj0 + 1, kh = k - kk0 + 1;
-  esirk_1d(ax0, ax1, ih, axh, currx);
-  esirk_1d(ay0, ay1, jh, ayh, curry);
-  esirk_1d(az0, az1, kh, azh, currz);
-#pragma unroll
-  for (int q = 0; q < 5; ++q) {
-    currx[q] = w * currx[q];
-    curry[q] = w * curry[q];
-    currz[q] = w * currz[q];
-    axh0[q] = 0.5 * axh[q];
-    axh1[q] = axh[q];
-    ayh0[q] = 0.5 * ayh[q];
-    ayh1[q] = ayh[q];
-  }
-#pragma unroll
-  for (int q = 1; q <= 3; ++q) {
-    axh0[q] = axh0[q] + ax0[q - 1];
-    axh1[q] = axh1[q] + 0.5 * ax0[q - 1];
-    ayh0[q] = ayh0[q] + ay0[q - 1];
-    ayh1[q] = ayh1[q] + 0.5 * ay0[q - 1];
-  }
-  const int x0 = ih < 1 ? ih : 1, x1 = (ih + 2) > 3 ? ih + 2 : 3;
-  const int y0 = jh < 1 ? jh : 1, y1 = (jh + 2) > 3 ? jh + 2 : 3;
-  const int z0 = kh < 1 ? kh : 1, z1 = (kh + 2) > 3 ? kh + 2 : 3;
-  const long long sy = g.n1p, sz = (long long)g.n1p * g.n2p;
-  // slot (i1, j1, k1) of the window of component c sits at base + i1 + sy j1 + sz k1
-  const long long bx0 = goff(g, ii0 - 2, jj0 - 2, kk0 - 1), bx1 = goff(g, ii0 - 2, jj0 - 2, k - 1);
-  const long long bz0 = goff(g, ii0 - 2, jj0 - 1, kk0 - 2), bz1 = goff(g, ii0 - 2, j - 1, kk0 - 2);
-  const bool samek = (k == kk0), samej = (j == jj0);
-  double* jx = jc;
-  double* jy = jc + g.ncell;
-  double* jz = jc + 2 * g.ncell;
-#pragma unroll
-  for (int k1 = 0; k1 <= 2; ++k1)
-#pragma unroll
-    for (int j1 = 0; j1 < 5; ++j1) {
-      if (j1 < y0 || j1 > y1) continue;
-      const double dvol = ayh0[j1] * az0[k1], dvolh = ayh1[j1] * az1[k1];
-      const double cvol = curry[j1] * az0[k1], cvolh = curry[j1] * az1[k1];
-#pragma unroll
-      for (int i1 = 0; i1 < 5; ++i1) {
-        if (i1 < x0 || i1 > x1) continue;
-        const long long o0 = bx0 + i1 + sy * j1 + sz * k1, o1 = bx1 + i1 + sy * j1 + sz * k1;
-        const double ax = dvol * currx[i1], bx = dvolh * currx[i1];
-        const double ay = axh0[i1] * cvol, by = axh1[i1] * cvolh;
-        if (samek) {
-          atomicAdd(&jx[o0], ax + bx);
-          atomicAdd(&jy[o0], ay + by);
-        } else {
-          atomicAdd(&jx[o0], ax);
-          atomicAdd(&jx[o1], bx);
-          atomicAdd(&jy[o0], ay);
-          atomicAdd(&jy[o1], by);
-        }
-      }
-    }
-#pragma unroll
-  for (int k1 = 0; k1 < 5; ++k1) {
-    if (k1 < z0 || k1 > z1) continue;
-#pragma unroll
-    for (int j1 = 0; j1 <= 2; ++j1) {
-      const double dvol = ay0[j1] * currz[k1], dvolh = ay1[j1] * currz[k1];
-#pragma unroll
-      for (int i1 = 0; i1 < 5; ++i1) {
-        if (i1 < x0 || i1 > x1) continue;
-        const long long o0 = bz0 + i1 + sy * j1 + sz * k1, o1 = bz1 + i1 + sy * j1 + sz * k1;
-        const double az = axh0[i1] * dvol, bz = axh1[i1] * dvolh;
-        if (samej) {
-          atomicAdd(&jz[o0], az + bz);
-        } else {
-          atomicAdd(&jz[o0], az);
-          atomicAdd(&jz[o1], bz);
-        }
-      }
-    }
-  }
-  return true;
-}
 
 // set_env_acc (src/particles/grid_part_connect.f90:414-615) ->
 // lpf_env_momenta (src/dynamics/boris_push.f90:170-223) ->
@@ -793,8 +698,7 @@ __global__ void __launch_bounds__(256) k_env_pos(EnvArgs a) {
       ncdef3d<SERIAL>(g, a.jc, xnl, xo, pp, wght, dt_lp * gam_inv);
       continue;
     }
-    const bool dep_ok = SERIAL ? esirkepov3d<true>(g, a.jc, xnl, xo, wght) : esirkepov3d_sum(g, a.jc, xnl, xo, wght);
-    if (!dep_ok) raise_err(a.err, AGPU_EBIT_INDEX);
+    if (!esirkepov3d<SERIAL>(g, a.jc, xnl, xo, wght)) raise_err(a.err, AGPU_EBIT_INDEX);
   }
 }
 

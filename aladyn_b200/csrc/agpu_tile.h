@@ -56,12 +56,21 @@ struct TileArgs64 {
   unsigned int* err;
 };
 
+// The envelope cycle's particle steps on the same tiles: the source scratch
+// av (F and its gradient) and the density.
+struct EnvTileArgs : TileArgs64 {
+  const double* av;
+  double* den;
+};
+
 TileGeo make_tiles(const Geo& g, int nx, int ny, int nz, bool fp32);
 int tile_push32(const TileArgs32& a, cudaStream_t st, int sms);
 int tile32_list_cap(int ndim);
 // the cubic shape extension (agpu_tile32c.cu)
 void tile_push32_cubic(const TileArgs32& a, cudaStream_t st);
 void tile_push64(const TileArgs64& a, cudaStream_t st);
+void env_acc_tile(const EnvTileArgs& a, cudaStream_t st);
+void env_pos_tile(const EnvTileArgs& a, cudaStream_t st);
 void hist_reset(int* hist, const int* tstart, const TileGeo& t, long long np, bool first, unsigned long long* pushed,
                 cudaStream_t st);
 

@@ -57,3 +57,36 @@ def test_fp64_tile_step(ndim, nx, ny, nz, n, how, pmax):
     ja, jb = dev.get_currents(), ora.get_currents()
     assert np.abs(ja - jb).max() <= 1e-12 * np.abs(jb).max()
 
+
+def env_step(cls, p, ep, rec, ebf, env0, nsteps):
+    d = cls(p)
+    d.env_enable(ep)
+    d.set_envelope(env0)
+    d.set_fields(ebf)
+    d.set_species(0, rec)
+    for it in range(1, nsteps + 1):
+        d.env_run(it * p.dt, it)
+    return d
+
+
+@pytest.mark.parametrize("ndim,nx,ny,nz,n,how", CASES)
+@pytest.mark.parametrize("pmax", [0.0, 2.0])
+def test_env_tile_steps(ndim, nx, ny, nz, n, how, pmax):
+    """Three envelope steps (the binning of one step serves the next): the
+    density and current sums reach every output, so 1e-12 of the largest
+    value (see above); the records are compared as sorted columns."""
+    from tests.test_envelope import env_case, numpy_init, pulse
+    p, g, ep = env_case(ndim, nx=nx, ny=ny, nz=nz, der_ord=2, cap=n + 16, w_sh=10)
+    env0 = numpy_init(p, pulse(p, a0=1.0, xc_frac=0.5, wx_frac=0.3, wy_frac=0.4))
+    rec, ebf = records(p, n, how, pmax), 0.02 * laser_fields(p)
+    rec[:, 2 * ndim] = pack_slot(np.full(n, -1), np.zeros(n), np.full(n, 0.01 / max(n / 1000, 1), np.float32))
+    dev = env_step(PicDevice, p, ep, rec, ebf, env0, 3)
+    ora = env_step(Oracle, p, ep, rec, ebf, env0, 3)
+    for f in ("get_envelope", "get_env_source", "get_fields", "get_currents"):
+        a, b = getattr(dev, f)(), getattr(ora, f)()
+        assert np.abs(a - b).max() <= 1e-12 * np.abs(b).max(), f
+    a, b = dev.get_species(0), ora.get_species(0)
+    assert a.shape == b.shape
+    for c in range(2 * ndim):
+        x, y = np.sort(a[:, c]), np.sort(b[:, c])
+        assert np.abs(x - y).max() <= 1e-12 * np.abs(y).max(), c
