@@ -149,7 +149,7 @@ struct CAcc {
   static constexpr int S = 128, RMAX = 16, ND = NDIM + 1;             // offsets and weight / gamma
   static constexpr int W_DEP = NF * FV, DOUBLES = W_DEP + NROW * ND * S;
   static constexpr int INTS = NROW * 32;
-  static constexpr size_t BYTES = sizeof(double) * DOUBLES + sizeof(int) * INTS + NROW * RMAX * 32;
+  static constexpr size_t BYTES = sizeof(double) * DOUBLES + sizeof(int) * INTS + NROW * (RMAX + 1) * 32;
 };
 
 // Density of one particle on its 3^NDIM nodes (set_env_density), for those
@@ -181,7 +181,8 @@ __global__ void __launch_bounds__(CAcc<NDIM>::NT, (NDIM == 3) ? 1 : 2) k_env_acc
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double* dep = smd + C::W_DEP + warp * ND * S;
   int* cnt = reinterpret_cast<int*>(smd + C::DOUBLES) + warp * 32;
-  unsigned char* idx = reinterpret_cast<unsigned char*>(smd + C::DOUBLES) + sizeof(int) * C::INTS + warp * RMAX * 32;
+  unsigned char* idx = reinterpret_cast<unsigned char*>(smd + C::DOUBLES) + sizeof(int) * C::INTS + warp * (RMAX + 1) * 32;
+  unsigned char* ord = idx + RMAX * 32;
 
   const int b = blockIdx.x, plane = a.t.ntx * a.t.nty;
   const int tx = b % a.t.ntx, ty = (b / a.t.ntx) % a.t.nty, zp = b / plane;
@@ -210,9 +211,14 @@ __global__ void __launch_bounds__(CAcc<NDIM>::NT, (NDIM == 3) ? 1 : 2) k_env_acc
 #pragma unroll 1
     for (int bq = 0; bq < S; bq += 32) {
       if (c0 + bq >= qend) break;
-      const int q = c0 + bq + lane, e = bq + lane;
-      if (q < qend) {
-        const int n = a.perm[q];
+      // lanes of the row's lower 16 nodes first (see tile64_step)
+      const int nact = min(32, qend - c0 - bq), e = bq + lane;
+      const int n0 = lane < nact ? a.perm[c0 + e] : 0;
+      double s;
+      const bool low = lane < nact && node_d(a.dx_inv * (a.x[n0] - a.xmn), s) < i0t + 16;
+      const int src = partition_lanes(low, ord);
+      const int n = __shfl_sync(0xffffffffu, n0, src);
+      if (src < nact) {
         const uint64_t sl = dbits(a.slot[n]);
         const double charge = (double)slot_charge(sl);
         const double wgh = (double)slot_wgh(sl);
@@ -383,7 +389,6 @@ __global__ void __launch_bounds__(CAcc<NDIM>::NT, (NDIM == 3) ? 1 : 2) k_env_acc
             a.pz[n] = pn[2];
             if (!(pn[0] == pn[0] && pn[1] == pn[1] && pn[2] == pn[2])) raise_err(a.err, AGPU_EBIT_NONFINITE);
           }
-          double s;
           node_d(xl, s);
           dep[e] = s;
           node_d(yl, s);

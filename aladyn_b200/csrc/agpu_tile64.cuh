@@ -60,7 +60,7 @@ struct C64 {
   static constexpr int DOUBLES = W_DEP + NROW * ND * S;
   // node counts; the group's record indices, then its movers; next histogram
   static constexpr int INTS = NROW * (32 + S) + NSUB;
-  static constexpr size_t BYTES = sizeof(double) * DOUBLES + sizeof(int) * INTS + NROW * RMAX * 32;
+  static constexpr size_t BYTES = sizeof(double) * DOUBLES + sizeof(int) * INTS + NROW * (RMAX + 1) * 32;
   static_assert(TX == 32 && S <= 256, "one x-row of 32 nodes per warp, list entries in one byte");
 };
 
@@ -73,6 +73,18 @@ __device__ __forceinline__ void cpa8z(void* sdst, const void* gsrc, bool valid) 
 __device__ __forceinline__ void cpa8(void* sdst, const void* gsrc) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(sdst);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(gsrc) : "memory");
+}
+
+// Source lane of each lane when the lanes with `low` set come first, both
+// parts in lane order; ord: 32 bytes of the warp's shared memory.
+__device__ __forceinline__ int partition_lanes(bool low, unsigned char* ord) {
+  const int lane = threadIdx.x & 31;
+  const unsigned m = __ballot_sync(0xffffffffu, low), lt = (1u << lane) - 1u;
+  ord[low ? __popc(m & lt) : __popc(m) + __popc(~m & lt)] = (unsigned char)lane;
+  __syncwarp();
+  const int src = ord[lane];
+  __syncwarp();
+  return src;
 }
 
 __device__ __forceinline__ void red64(double* p, double v) {
@@ -297,7 +309,8 @@ __device__ __forceinline__ void tile64_step(const typename P::Args& a) {
   double* dep = smd + C::W_DEP + warp * ND * S;
   int* cnt = sInt + warp * (32 + S);
   int* mov = cnt + 32;
-  unsigned char* idx = reinterpret_cast<unsigned char*>(sHist + C::NSUB) + warp * RMAX * 32;
+  unsigned char* idx = reinterpret_cast<unsigned char*>(sHist + C::NSUB) + warp * (RMAX + 1) * 32;
+  unsigned char* ord = idx + RMAX * 32;
 
   stage64<C::NF, C::FX, C::FY, C::FZ, C::NROW>(sF, g, i0t - C::LO, j0t - C::LO, (NDIM == 3) ? k0t - C::LO : 1,
                                                [&](int c) { return P::comp(a, c); });
@@ -339,15 +352,21 @@ __device__ __forceinline__ void tile64_step(const typename P::Args& a) {
       if (b == 0) asm volatile("cp.async.wait_group %0;\n" ::"n"(S / 32 - 1) : "memory");
       else if (b == 32) asm volatile("cp.async.wait_group %0;\n" ::"n"(S / 32 - 2) : "memory");
       else asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-      const int q = c0 + b + lane;
+      __syncwarp();  // the batch's records, copied by its other lanes too
+      // lanes of the row's lower 16 nodes first: an 8-byte shared load serves
+      // 16 lanes at a time, and nodes i and i + 16 share banks (the records of
+      // a batch stay the same, so global accesses stay coalesced)
+      const int nact = min(32, qend - c0 - b);
+      double s_;
+      const bool low = lane < nact && node_d(a.dx_inv * (dep[b + lane] - a.xmn), s_) < i0t + 16;
+      const int src = partition_lanes(low, ord);
       int meta = -1;  // mover list entry
-      if (q < qend) {
-        const int e = b + lane;
+      if (src < nact) {
+        const int e = b + src;
         const int p = mov[e];  // this batch's entries are read before its movers are listed
         // (the record is read again after the gather instead of held through it)
         const double xo[3] = {a.dx_inv * (dep[e] - a.xmn), a.dy_inv * (dep[S + e] - a.ymn),
                               (NDIM == 3) ? a.dz_inv * (dep[2 * S + e] - a.zmn) : 0.};
-        double s_;
         const int fx = node_d(xo[0], s_) - i0t, fy = node_d(xo[1], s_) - j0t, fz = (NDIM == 3) ? node_d(xo[2], s_) - k0t : 0;
         if ((unsigned)fx >= (unsigned)TX || fy != wy || (NDIM == 3 && fz != wz)) {
           raise_err(a.err, AGPU_EBIT_INDEX);  // not binned in this row: drop it
