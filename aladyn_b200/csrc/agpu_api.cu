@@ -132,15 +132,20 @@ struct agpu_handle {
   int* tstart[4] = {nullptr, nullptr, nullptr, nullptr};
   int* cursor = nullptr;
   int* scan_tmp = nullptr;
-  // staging of window-injection records for the split form (kept between
-  // calls: a per-call device allocation of hundreds of MB can take longer
-  // than the step)
-  double* inj_stage = nullptr;
-  long long inj_stage_recs = 0;
+  // FP64 staging of host transfers (grown up to STAGE_MAX doubles and kept:
+  // a device allocation and its release in every call took 2 to 8 ms beside
+  // steps of 0.1 to 2 ms); larger arrays pass through it in chunks, in order
+  // on the handle's stream
+  double* stage = nullptr;
+  long long stage_n = 0;
   bool binned[4] = {false, false, false, false};
   long long nalive[4] = {0, 0, 0, 0};  // np minus removed records still stored
   // deferred counts: tiled steps leave the alive counts and the error word
   // on the device; refresh_counts reads them at the next synchronisation
+  // pend: alive counts of this step's tiled pushes still on their way to the
+  // host (pend[ic] = the count before the push, -1: none); settle_counts
+  // reads them with the step's one synchronisation
+  long long pend[4] = {-1, -1, -1, -1};
   bool defer = false;
   bool stale[4] = {false, false, false, false};
   // step graph (deferred mode): the launches of a step between window
@@ -178,6 +183,22 @@ int dmalloc(void** p, size_t bytes) {
     *p = nullptr;
     return AGPU_E_NOMEM;
   }
+  return 0;
+}
+
+// The staging buffer, at least min(n, STAGE_MAX) doubles.
+constexpr long long STAGE_MAX = 1ll << 23;
+int stage_grow(agpu_handle* h, long long n) {
+  n = std::min(n, STAGE_MAX);
+  if (h->stage_n >= n) return 0;
+  if (h->stage) {
+    cudaStreamSynchronize(h->st);
+    cudaFree(h->stage);
+  }
+  h->stage = nullptr;
+  h->stage_n = 0;
+  if (dmalloc((void**)&h->stage, sizeof(double) * n)) return AGPU_E_NOMEM;
+  h->stage_n = n;
   return 0;
 }
 
@@ -259,7 +280,7 @@ int free_all(agpu_handle* h) {
   }
   cudaFree(h->cursor);
   cudaFree(h->scan_tmp);
-  cudaFree(h->inj_stage);
+  cudaFree(h->stage);
   cudaFree(h->env);
   cudaFree(h->env_av);
   cudaFree(h->env_den);
@@ -317,6 +338,22 @@ int refresh_counts(agpu_handle* h) {
       h->stale[ic] = false;
     }
   CK(cudaMemsetAsync(h->d_cnt, 0, sizeof(Counters), h->st));
+  return 0;
+}
+
+// Counts of the step's tiled pushes, not deferred: one synchronisation for
+// all of them, where the counts are first needed or at the end of the step.
+int settle_counts(agpu_handle* h, agpu_step_out* out) {
+  bool any = false;
+  for (int ic = 0; ic < 4; ++ic) any = any || h->pend[ic] >= 0;
+  if (!any) return 0;
+  if (int rc = read_counters(h)) return rc;
+  for (int ic = 0; ic < 4; ++ic)
+    if (h->pend[ic] >= 0) {
+      h->nalive[ic] = h->h_cnt->alive4[ic];
+      out->removed[ic] += h->pend[ic] - h->nalive[ic];
+      h->pend[ic] = -1;
+    }
   return 0;
 }
 
@@ -587,7 +624,7 @@ void tile_args64(const agpu_handle* h, int ic, int initial_time, TileArgs64& a) 
 // Tiled gather + push + deposit of species ic, then the next binning from
 // the keys the kernel wrote.  Removed particles stay stored (key nkeys)
 // until the next compaction.
-int tiled_push(agpu_handle* h, int ic, int initial_time, agpu_step_out* out) {
+int tiled_push(agpu_handle* h, int ic, int initial_time) {
   const agpu_params& p = h->p;
   if (!h->binned[ic]) {
     ph_begin(h, PH_SORT);
@@ -645,11 +682,9 @@ int tiled_push(agpu_handle* h, int ic, int initial_time, agpu_step_out* out) {
     ph_end(h, PH_SORT);
     return 0;
   }
-  CK(cudaMemcpyAsync(&h->d_cnt->alive, h->tstart[ic] + h->tg.nkeys, sizeof(int), cudaMemcpyDeviceToDevice, h->st));
-  if (int rc = read_counters(h)) return rc;
+  CK(cudaMemcpyAsync(&h->d_cnt->alive4[ic], h->tstart[ic] + h->tg.nkeys, sizeof(int), cudaMemcpyDeviceToDevice, h->st));
+  h->pend[ic] = alive0;
   ph_end(h, PH_SORT);
-  h->nalive[ic] = h->h_cnt->alive;
-  out->removed[ic] += alive0 - h->nalive[ic];
   return 0;
 }
 
@@ -1088,7 +1123,7 @@ int agpu_create(const agpu_params* params, agpu_handle** out) {
     rc |= dmalloc((void**)&h->d_diag, sizeof(double) * 64);
     rc |= dmalloc((void**)&h->d_envar, sizeof(double) * (16 + AGPU_NE));
     if (h->fp32) {
-      // every chunk beyond a tile's first holds LIST_CAP particles
+      // every chunk beyond a tile's first holds a full chunk of particles
       h->tile_work_cap = (int)(capmax / tile32_list_cap(p.ndim)) + 16;
       rc |= dmalloc((void**)&h->tile_work, sizeof(int) * 2 * (size_t)h->tile_work_cap);
       rc |= dmalloc((void**)&h->tile_work_n, 2 * sizeof(unsigned int));
@@ -1162,12 +1197,13 @@ int agpu_set_fields(agpu_handle* h, const double* ebf, int32_t n1p, int32_t n2p,
   if (!h->fp32) {
     CK(cudaMemcpyAsync(h->ebf, ebf, sizeof(double) * n, cudaMemcpyHostToDevice, h->st));
   } else {
-    double* stage = nullptr;
-    if (dmalloc((void**)&stage, sizeof(double) * n)) return AGPU_E_NOMEM;
-    cudaMemcpyAsync(stage, ebf, sizeof(double) * n, cudaMemcpyHostToDevice, h->st);
-    f64_to_f32(stage, h->ebf32, (long long)n, h->st, h->sms);
-    cudaStreamSynchronize(h->st);
-    cudaFree(stage);
+    if (int rc = stage_grow(h, (long long)n)) return rc;
+    for (size_t q = 0; q < n; q += STAGE_MAX) {
+      const size_t m = std::min(n - q, (size_t)STAGE_MAX);
+      CK(cudaMemcpyAsync(h->stage, ebf + q, sizeof(double) * m, cudaMemcpyHostToDevice, h->st));
+      f64_to_f32(h->stage, h->ebf32 + q, (long long)m, h->st, h->sms);
+    }
+    CK(cudaGetLastError());
   }
   CK(cudaStreamSynchronize(h->st));
   h->fields_set = true;
@@ -1182,12 +1218,12 @@ int agpu_get_fields(agpu_handle* h, double* ebf, int32_t n1p, int32_t n2p, int32
   if (!h->fp32) {
     CK(cudaMemcpyAsync(ebf, h->ebf, sizeof(double) * n, cudaMemcpyDeviceToHost, h->st));
   } else {
-    double* stage = nullptr;
-    if (dmalloc((void**)&stage, sizeof(double) * n)) return AGPU_E_NOMEM;
-    f32_to_f64(h->ebf32, stage, (long long)n, h->st, h->sms);
-    cudaMemcpyAsync(ebf, stage, sizeof(double) * n, cudaMemcpyDeviceToHost, h->st);
-    cudaStreamSynchronize(h->st);
-    cudaFree(stage);
+    if (int rc = stage_grow(h, (long long)n)) return rc;
+    for (size_t q = 0; q < n; q += STAGE_MAX) {
+      const size_t m = std::min(n - q, (size_t)STAGE_MAX);
+      f32_to_f64(h->ebf32 + q, h->stage, (long long)m, h->st, h->sms);
+      CK(cudaMemcpyAsync(ebf + q, h->stage, sizeof(double) * m, cudaMemcpyDeviceToHost, h->st));
+    }
   }
   CK(cudaStreamSynchronize(h->st));
   return 0;
@@ -1197,25 +1233,21 @@ int agpu_get_currents(agpu_handle* h, double* jc, int32_t n1p, int32_t n2p, int3
   if (!h || !jc) return AGPU_E_ARG;
   const Geo& g = h->g;
   if (n1p != g.n1p || n2p != g.n2p || n3p != g.n3p || nc != g.nc) return AGPU_E_ARG;
-  size_t n = (size_t)g.ncell * g.nc;
-  if (!h->fp32) {
-    CK(cudaMemcpyAsync(jc, h->jc, sizeof(double) * n, cudaMemcpyDeviceToHost, h->st));
-  } else {
-    double* stage = nullptr;
-    if (dmalloc((void**)&stage, sizeof(double) * n)) return AGPU_E_NOMEM;
-    f32pair_to_f64(h->jhi, h->jlo, stage, (long long)n, h->st, h->sms);
-    cudaMemcpyAsync(jc, stage, sizeof(double) * n, cudaMemcpyDeviceToHost, h->st);
-    cudaStreamSynchronize(h->st);
-    cudaFree(stage);
+  // curr = djc(i) * curr (curr_and_fields_util.f90:111-115), whole array,
+  // scaled on the way out
+  const size_t n = (size_t)g.ncell;
+  if (int rc = stage_grow(h, (long long)n)) return rc;
+  for (int c = 0; c < g.nc; ++c) {
+    const double d = h->p.iform < 2 ? h->p.djc[c] : 1.0;
+    for (size_t q = 0; q < n; q += STAGE_MAX) {
+      const size_t m = std::min(n - q, (size_t)STAGE_MAX), o = n * c + q;
+      if (h->fp32) scaled_out(nullptr, h->jhi + o, h->jlo + o, h->stage, d, (long long)m, h->st, h->sms);
+      else scaled_out(h->jc + o, nullptr, nullptr, h->stage, d, (long long)m, h->st, h->sms);
+      CK(cudaGetLastError());
+      CK(cudaMemcpyAsync(jc + o, h->stage, sizeof(double) * m, cudaMemcpyDeviceToHost, h->st));
+    }
   }
   CK(cudaStreamSynchronize(h->st));
-  // curr = djc(i) * curr (curr_and_fields_util.f90:111-115), whole array
-  if (h->p.iform < 2)
-    for (int i = 0; i < h->p.ndim; ++i) {
-      double d = h->p.djc[i];
-      double* c = jc + (size_t)g.ncell * i;
-      for (size_t q = 0; q < (size_t)g.ncell; ++q) c[q] = d * c[q];
-    }
   if (h->str) {
     // the stretched metric on the interior (curr_and_fields_util.f90:120-150)
     const int ny = h->p.ny;
@@ -1252,14 +1284,16 @@ int agpu_set_species(agpu_handle* h, int32_t ic, const double* part, int64_t ld,
       CK(cudaMemcpy2DAsync(h->part[ic], sizeof(double) * h->cap[ic], part, sizeof(double) * ld, sizeof(double) * np, ndv,
                            cudaMemcpyHostToDevice, h->st));
   } else if (np > 0) {
-    double* stage = nullptr;
-    if (dmalloc((void**)&stage, sizeof(double) * np * ndv)) return AGPU_E_NOMEM;
-    cudaMemcpy2DAsync(stage, sizeof(double) * np, part, sizeof(double) * ld, sizeof(double) * np, ndv, cudaMemcpyHostToDevice,
-                      h->st);
-    rec_to_split(stage, np, np, h->sp[ic].view(), 0, h->g, h->p.xmn, h->p.ymn, h->p.zmn, h->p.dx_inv, h->p.dy_inv, h->p.dz_inv,
-                 h->st, h->sms);
-    cudaStreamSynchronize(h->st);
-    cudaFree(stage);
+    if (int rc = stage_grow(h, np * ndv)) return rc;
+    const long long chunk = STAGE_MAX / ndv;
+    for (long long q = 0; q < np; q += chunk) {
+      const long long m = std::min<long long>(np - q, chunk);
+      CK(cudaMemcpy2DAsync(h->stage, sizeof(double) * m, part + q, sizeof(double) * ld, sizeof(double) * m, ndv,
+                           cudaMemcpyHostToDevice, h->st));
+      rec_to_split(h->stage, m, m, h->sp[ic].view(), q, h->g, h->p.xmn, h->p.ymn, h->p.zmn, h->p.dx_inv, h->p.dy_inv,
+                   h->p.dz_inv, h->st, h->sms);
+      CK(cudaGetLastError());
+    }
   }
   CK(cudaStreamSynchronize(h->st));
   h->np[ic] = np;
@@ -1284,13 +1318,26 @@ int agpu_get_species(agpu_handle* h, int32_t ic, double* part, int64_t ld, int64
     CK(cudaMemcpy2DAsync(part, sizeof(double) * ld, h->part[ic], sizeof(double) * h->cap[ic], sizeof(double) * n, ndv,
                          cudaMemcpyDeviceToHost, h->st));
   } else {
-    double* stage = nullptr;
-    if (dmalloc((void**)&stage, sizeof(double) * n * ndv)) return AGPU_E_NOMEM;
-    split_to_rec(h->sp[ic].view(), n, stage, n, h->g, h->p.xmn, h->p.ymn, h->p.zmn, h->p.dx, h->p.dy, h->p.dz, h->st, h->sms);
-    cudaMemcpy2DAsync(part, sizeof(double) * ld, stage, sizeof(double) * n, sizeof(double) * n, ndv, cudaMemcpyDeviceToHost,
-                      h->st);
-    cudaStreamSynchronize(h->st);
-    cudaFree(stage);
+    if (int rc = stage_grow(h, n * ndv)) return rc;
+    const long long chunk = STAGE_MAX / ndv;
+    for (long long q = 0; q < n; q += chunk) {
+      const long long m = std::min(n - q, chunk);
+      Part32View v = h->sp[ic].view();
+      v.cell += q;
+      v.ox += q;
+      v.oy += q;
+      v.px += q;
+      v.py += q;
+      if (v.oz) {
+        v.oz += q;
+        v.pz += q;
+      }
+      v.slot += q;
+      split_to_rec(v, m, h->stage, m, h->g, h->p.xmn, h->p.ymn, h->p.zmn, h->p.dx, h->p.dy, h->p.dz, h->st, h->sms);
+      CK(cudaGetLastError());
+      CK(cudaMemcpy2DAsync(part + q, sizeof(double) * ld, h->stage, sizeof(double) * m, sizeof(double) * m, ndv,
+                           cudaMemcpyDeviceToHost, h->st));
+    }
   }
   CK(cudaStreamSynchronize(h->st));
   return 0;
@@ -1720,10 +1767,10 @@ static int step_impl(agpu_handle* h, int32_t iter, double t, int32_t initial_tim
   out->ion_field_max = -1.0;
   agpu_params& p = h->p;
   int rc = 0;
+  for (int ic = 0; ic < 4; ++ic) h->pend[ic] = -1;
   if (h->defer) {
-    // keep the error word and the push count accumulating on the device
-    CK(cudaMemsetAsync(&h->d_cnt->removed, 0, sizeof(unsigned long long), h->st));
-    CK(cudaMemsetAsync(&h->d_cnt->fmax, 0, sizeof(double), h->st));
+    // the error word and the push count keep accumulating on the device (the
+    // untiled push and the ionization clear their own counters)
     if (p.ionz_lev > 0)
       if (int rc_ = refresh_counts(h)) return rc_;
   } else {
@@ -1759,11 +1806,14 @@ static int step_impl(agpu_handle* h, int32_t iter, double t, int32_t initial_tim
       continue;
     }
     if (tiled(h, ic)) {
-      if (int rc_ = tiled_push(h, ic, initial_time, out)) return rc_;
-      if (sort_step(h, iter))
+      if (int rc_ = tiled_push(h, ic, initial_time)) return rc_;
+      if (sort_step(h, iter)) {
+        if (int rc_ = settle_counts(h, out)) return rc_;
         if (int rc_ = reorder_records(h, ic)) return rc_;
+      }
       continue;
     }
+    if (int rc_ = settle_counts(h, out)) return rc_;
     if (int rc_ = drop_removed(h, ic)) return rc_;
     np = h->np[ic];
     CK(cudaMemsetAsync(&h->d_cnt->removed, 0, sizeof(unsigned long long), h->st));
@@ -1897,9 +1947,14 @@ static int step_impl(agpu_handle* h, int32_t iter, double t, int32_t initial_tim
   // current fold (x, y[, z] faces; hi and lo in the split form) + the Yee kernels
   h->timers.launches_total += ((p.ndim == 3) ? 3 : 2) * (h->fp32 ? 2 : 1) + (fused ? 1 : 6) + xadv_launches(h);
   h->timers.yee_cells += (long long)p.nx * p.ny * (p.ndim == 3 ? p.nz : 1);
-  // lp_run: moving window, or the comoving frame's coordinate shift
+  // lp_run: moving window, or the comoving frame's coordinate shift.  The
+  // counts come over once, after the last kernel of a plain step or before
+  // the compaction of a window step (whose errors are read again).
+  const bool pending = !h->defer && h->pend[0] + h->pend[1] + h->pend[2] + h->pend[3] > -4;
+  if (int rc_ = settle_counts(h, out)) return rc_;
+  const bool event = p.w_sh > 0 && p.w_speed != 0.0 && t >= p.wi_time && t < p.wf_time && iter % p.w_sh == 0;
   if (int rc_ = window_or_comoving(h, iter, t, out)) return rc_;
-  if (!h->defer)
+  if (!h->defer && (event || !pending))
     if (int rc_ = read_counters(h)) return rc_;
   // deferred mode: the counts of the last synchronisation point
   for (int ic = 0; ic < 4; ++ic) out->np[ic] = h->binned[ic] ? h->nalive[ic] : h->np[ic];
@@ -2117,23 +2172,13 @@ int agpu_window_inject(agpu_handle* h, int32_t ic, const double* part, int64_t l
     CK(cudaMemcpy2DAsync(h->part[ic] + h->np[ic], sizeof(double) * h->cap[ic], part, sizeof(double) * ld, sizeof(double) * n,
                          ndv, cudaMemcpyHostToDevice, h->st));
   } else {
-    // chunks of at most 2^20 records through a staging buffer kept in the
-    // handle (allocated on the first call, grown up to the chunk size)
-    const long long chunk_max = 1ll << 20;
-    const long long chunk = n < chunk_max ? n : chunk_max;
-    if (h->inj_stage_recs < chunk) {
-      CK(cudaStreamSynchronize(h->st));
-      cudaFree(h->inj_stage);
-      h->inj_stage = nullptr;
-      h->inj_stage_recs = 0;
-      if (dmalloc((void**)&h->inj_stage, sizeof(double) * chunk * ndv)) return AGPU_E_NOMEM;
-      h->inj_stage_recs = chunk;
-    }
+    if (int rc = stage_grow(h, n * ndv)) return rc;
+    const long long chunk = STAGE_MAX / ndv;
     for (long long q0 = 0; q0 < n; q0 += chunk) {
-      const long long m = (n - q0) < chunk ? (n - q0) : chunk;
-      CK(cudaMemcpy2DAsync(h->inj_stage, sizeof(double) * m, part + q0, sizeof(double) * ld, sizeof(double) * m, ndv,
+      const long long m = std::min<long long>(n - q0, chunk);
+      CK(cudaMemcpy2DAsync(h->stage, sizeof(double) * m, part + q0, sizeof(double) * ld, sizeof(double) * m, ndv,
                            cudaMemcpyHostToDevice, h->st));
-      rec_to_split(h->inj_stage, m, m, h->sp[ic].view(), h->np[ic] + q0, h->g, h->p.xmn, h->p.ymn, h->p.zmn, h->p.dx_inv,
+      rec_to_split(h->stage, m, m, h->sp[ic].view(), h->np[ic] + q0, h->g, h->p.xmn, h->p.ymn, h->p.zmn, h->p.dx_inv,
                    h->p.dy_inv, h->p.dz_inv, h->st, h->sms);
       CK(cudaGetLastError());
     }

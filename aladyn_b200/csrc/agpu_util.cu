@@ -465,9 +465,10 @@ __global__ void k_f32_to_f64(const float* a, double* b, long long n) {
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
     b[q] = (double)a[q];
 }
-__global__ void k_f32pair_to_f64(const float* hi, const float* lo, double* b, long long n) {
+// out = d * (j64, or hi + lo when j64 is null)
+__global__ void k_scaled_out(const double* j64, const float* hi, const float* lo, double* out, double d, long long n) {
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
-    b[q] = (double)hi[q] + (double)lo[q];
+    out[q] = d * (j64 ? j64[q] : (double)hi[q] + (double)lo[q]);
 }
 void f64_to_f32(const double* a, float* b, long long n, cudaStream_t st, int sms) {
   k_f64_to_f32<<<grid_for(n, 256, sms, 16), 256, 0, st>>>(a, b, n);
@@ -475,8 +476,9 @@ void f64_to_f32(const double* a, float* b, long long n, cudaStream_t st, int sms
 void f32_to_f64(const float* a, double* b, long long n, cudaStream_t st, int sms) {
   k_f32_to_f64<<<grid_for(n, 256, sms, 16), 256, 0, st>>>(a, b, n);
 }
-void f32pair_to_f64(const float* hi, const float* lo, double* b, long long n, cudaStream_t st, int sms) {
-  k_f32pair_to_f64<<<grid_for(n, 256, sms, 16), 256, 0, st>>>(hi, lo, b, n);
+void scaled_out(const double* j64, const float* hi, const float* lo, double* out, double d, long long n, cudaStream_t st,
+                int sms) {
+  k_scaled_out<<<grid_for(n, 256, sms, 16), 256, 0, st>>>(j64, hi, lo, out, d, n);
 }
 
 // ============================================================================

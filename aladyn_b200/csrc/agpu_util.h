@@ -88,7 +88,8 @@ void split_to_rec(const Part32View& p, long long n, double* rec, long long ld, c
                   double dx, double dy, double dz, cudaStream_t st, int sms);
 void f64_to_f32(const double* a, float* b, long long n, cudaStream_t st, int sms);
 void f32_to_f64(const float* a, double* b, long long n, cudaStream_t st, int sms);
-void f32pair_to_f64(const float* hi, const float* lo, double* b, long long n, cudaStream_t st, int sms);
+void scaled_out(const double* j64, const float* hi, const float* lo, double* out, double d, long long n, cudaStream_t st,
+                int sms);
 void laser64(const LaserArgs& a, double* ebf, const Geo& g, cudaStream_t st, int sms);
 void field_diag64(const double* ebf, const Geo& g, double dvol, double* out_e, double* out_max, cudaStream_t st, int sms);
 void field_diag32(const float* ebf, const Geo& g, double dvol, double* out_e, double* out_max, cudaStream_t st, int sms);
