@@ -633,7 +633,7 @@ int tiled_push(agpu_handle* h, int ic, int initial_time) {
     if (rc) return rc;
   }
   const long long alive0 = h->nalive[ic];
-  hist_reset(h->hist[ic], h->tstart[ic], h->tg, h->np[ic], false, h->defer ? &h->d_cnt->pushed : nullptr, h->st);
+  hist_reset(h->hist[ic], h->tstart[ic], h->tg, h->np[ic], h->defer ? &h->d_cnt->pushed : nullptr, h->tile_work_n, h->st);
   ph_begin(h, PH_PUSH);
   if (h->fp32) {
     TileArgs32 a;
@@ -1649,6 +1649,8 @@ int agpu_x_step_many(agpu_handle** hs, int32_t n, agpu_x_ws* w) {
   const int ndim = hs[0]->p.ndim;
   long long max_cells = 1, max_faces = 1, max_np = 1;
   int total = 0;
+  int max_keys = 0;
+  bool bds = true;
   for (int i = 0; i < n; ++i) {
     agpu_handle* h = hs[i];
     if (h->p.ndim != ndim) return AGPU_E_ARG;
@@ -1679,6 +1681,7 @@ int agpu_x_step_many(agpu_handle** hs, int32_t n, agpu_x_ws* w) {
     a.work_cap = 0;
     m.ebf = h->ebf32;
     m.yc = yee_coef(p);
+    bds = bds && m.yc.se2 == 0.0;
     m.cursor = h->cursor;
     m.pushed = &h->d_cnt->pushed;
     m.removed = &h->d_cnt->removed;
@@ -1692,6 +1695,7 @@ int agpu_x_step_many(agpu_handle** hs, int32_t n, agpu_x_ws* w) {
     max_cells = std::max(max_cells, std::max(cells, g.ncell * g.nc));
     max_faces = std::max(max_faces, faces * g.nf);
     max_np = std::max(max_np, h->np[0]);
+    max_keys = std::max(max_keys, h->tg.nkeys);
   }
   w->h_off[n] = total;
   auto blocks = [](long long work, int cap) { return (int)std::max(1LL, std::min<long long>((work + 255) / 256, cap)); };
@@ -1702,12 +1706,13 @@ int agpu_x_step_many(agpu_handle** hs, int32_t n, agpu_x_ws* w) {
   pl.gx_cells = blocks(max_cells, 64);
   pl.gx_faces = blocks(max_faces, 16);
   pl.gx_parts = blocks(max_np, 128);
+  pl.bds = bds ? 1 : 0;
+  pl.max_keys = max_keys;
   cudaStream_t st = w->st;
   CK(cudaMemcpyAsync(w->d_desc, w->h_desc, sizeof(MultiInst) * n, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(w->d_off, w->h_off, sizeof(int) * (n + 1), cudaMemcpyHostToDevice, st));
   int launches = 0;
   multi_pre32(w->d_desc, pl, st, &launches);
-  multi_field_bd32(w->d_desc, pl, st, &launches);
   multi_tile32(w->d_desc, w->d_off, pl, st, &launches);
   multi_bin32(w->d_desc, pl, st, &launches);
   multi_fields32(w->d_desc, pl, st, &launches);
@@ -1781,7 +1786,7 @@ static int step_impl(agpu_handle* h, int32_t iter, double t, int32_t initial_tim
   if (h->fp32) field_bd32(Dev32{h->g, h->ebf32, h->jhi, h->jlo}, h->st, h->sms);
   else field_bd64(Dev64{h->g, h->ebf, h->jc}, h->st, h->sms);
   CK(cudaGetLastError());
-  h->timers.launches_total += (p.ndim == 3) ? 3 : 2;
+  h->timers.launches_total += 1;
   if (int rc_ = halo_call(h, AGPU_HALO_FIELDS, -1)) return rc_;
   ph_end(h, PH_YEE);
   // ionization
@@ -1944,8 +1949,8 @@ static int step_impl(agpu_handle* h, int32_t iter, double t, int32_t initial_tim
   CK(cudaGetLastError());
   ph_end(h, PH_YEE);
   h->timers.launches_yee += 1;
-  // current fold (x, y[, z] faces; hi and lo in the split form) + the Yee kernels
-  h->timers.launches_total += ((p.ndim == 3) ? 3 : 2) * (h->fp32 ? 2 : 1) + (fused ? 1 : 6) + xadv_launches(h);
+  // current fold + the Yee kernels
+  h->timers.launches_total += 1 + (fused ? 1 : yee_launches(c, h->dd || h->xadv.tmp)) + xadv_launches(h);
   h->timers.yee_cells += (long long)p.nx * p.ny * (p.ndim == 3 ? p.nz : 1);
   // lp_run: moving window, or the comoving frame's coordinate shift.  The
   // counts come over once, after the last kernel of a plain step or before
@@ -2365,7 +2370,7 @@ int agpu_env_run(agpu_handle* h, int32_t iter, double t, agpu_step_out* out) {
     tile_args64(h, ic, 0, ta);
     ta.av = h->env_av;
     ta.den = h->env_den;
-    hist_reset(h->hist[ic], h->tstart[ic], h->tg, h->np[ic], false, nullptr, h->st);
+    hist_reset(h->hist[ic], h->tstart[ic], h->tg, h->np[ic], nullptr, nullptr, h->st);
   }
   // set_env_acc, lpf_env_momenta, set_env_density (jc(:,:,:,1) = 0 first)
   CK(cudaMemsetAsync(h->env_den, 0, sizeof(double) * c3, h->st));
@@ -2417,7 +2422,7 @@ int agpu_env_run(agpu_handle* h, int32_t iter, double t, agpu_step_out* out) {
   CK(cudaGetLastError());
   ph_end(h, PH_YEE);
   h->timers.launches_yee += 1;
-  h->timers.launches_total += ((p.ndim == 3) ? 3 : 2) + 6 + xadv_launches(h);
+  h->timers.launches_total += 1 + yee_launches(yee_coef(p), h->xadv.tmp != nullptr) + xadv_launches(h);
   h->timers.yee_cells += (long long)p.nx * p.ny * (p.ndim == 3 ? p.nz : 1);
   if ((rc = window_or_comoving(h, iter, t, out, true))) return rc;
   if (int rc_ = read_counters(h)) return rc_;

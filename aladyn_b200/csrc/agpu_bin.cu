@@ -51,41 +51,14 @@ __global__ void k_keys_abs(const double* x, const double* y, const double* z, lo
   }
 }
 
-// Exclusive scan of hist[0..nb) into start[0..nb], one block.
-__device__ void d_scan_int(const int* hist, int nb, int* start) {
-  __shared__ long long part[1024];
-  int per = (nb + blockDim.x - 1) / blockDim.x;
-  int lo = threadIdx.x * per, hi = min(lo + per, nb);
-  long long s = 0;
-  for (int b = lo; b < hi; ++b) s += hist[b];
-  part[threadIdx.x] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    long long run = 0;
-    for (int q = 0; q < (int)blockDim.x; ++q) {
-      long long v = part[q];
-      part[q] = run;
-      run += v;
-    }
-    start[nb] = (int)run;
-  }
-  __syncthreads();
-  long long run = part[threadIdx.x];
-  for (int b = lo; b < hi; ++b) {
-    start[b] = (int)run;
-    run += hist[b];
-  }
-}
-__global__ void k_scan_int(const int* hist, int nb, int* start) { d_scan_int(hist, nb, start); }
-
-// perm[start[key] + rank] = n, ranks from warp-aggregated cursors.  Each warp
+// perm[cursor[key]++] = n with warp-aggregated cursors (which start at the
+// keys' first slots).  Each warp
 // takes SC_U consecutive runs of 32 records per pass, so that SC_U cursor
 // atomics (one round trip to L2 each) are in flight together; the lanes of
 // a run with one key get consecutive slots in lane order.  Warp-uniform loop
 // (blockDim a multiple of 32).
 constexpr int SC_U = 4;
-__device__ void d_perm_scatter(const int* key, long long np, const int* start, int* cursor, int* perm, long long bid_,
-                               long long nb_) {
+__device__ void d_perm_scatter(const int* key, long long np, int* cursor, int* perm, long long bid_, long long nb_) {
   const int lane = threadIdx.x & 31;
   const long long warp = (bid_ * (long long)blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = (nb_ * (long long)blockDim.x) >> 5;
@@ -107,12 +80,12 @@ __device__ void d_perm_scatter(const int* key, long long np, const int* start, i
 #pragma unroll
     for (int u = 0; u < SC_U; ++u) {
       const int bb = __shfl_sync(0xffffffffu, b[u], lead[u]);
-      if (kk[u] >= 0) perm[start[kk[u]] + bb + rank[u]] = (int)(base + u * 32 + lane);
+      if (kk[u] >= 0) perm[bb + rank[u]] = (int)(base + u * 32 + lane);
     }
   }
 }
-__global__ void k_perm_scatter(const int* key, long long np, const int* start, int* cursor, int* perm) {
-  d_perm_scatter(key, np, start, cursor, perm, blockIdx.x, gridDim.x);
+__global__ void k_perm_scatter(const int* key, long long np, int* cursor, int* perm) {
+  d_perm_scatter(key, np, cursor, perm, blockIdx.x, gridDim.x);
 }
 
 void bin_keys_split(const int* cell, const float* ox, const float* oy, const float* oz, long long np, const Geo& g,
@@ -126,62 +99,74 @@ void bin_keys_abs(const double* x, const double* y, const double* z, long long n
   if (np <= 0) return;
   k_keys_abs<<<grid_for(np, 256, sms, 16), 256, 0, st>>>(x, y, z, np, g, t, xmn, ymn, zmn, dxi, dyi, dzi, key, hist, err);
 }
-// ---- exclusive scan of many bins: block sums, a scan of the block sums,
-// then each block's scan offset by its block's start -------------------------
+// ---- exclusive scan of the histogram ------------------------------------
+// start[i] = cursor[i] = sum of hist[0..i), start[n] = total.  A block scans
+// SCAN_BLOCK bins and finds its first value itself, by adding what precedes
+// it: up to SCAN_ONE bins straight from the histogram (one launch; the last
+// block reads 256 KB from L2, about 3 us), beyond that from the blocks' sums
+// (two launches).  The earlier scan of the block sums by one serial block
+// was a launch of its own of 9 us on every grid.
 constexpr int SCAN_ITEMS = 16, SCAN_THREADS = 256, SCAN_BLOCK = SCAN_ITEMS * SCAN_THREADS;
+constexpr int SCAN_ONE = 16 * SCAN_BLOCK;
 
-__device__ __forceinline__ int block_exclusive_sum(int v, int* s_warp, int* total) {
+// Sum over the block of v and this thread's exclusive prefix.
+__device__ __forceinline__ int block_exclusive_sum(int v, int* total) {
+  __shared__ int s_warp[SCAN_THREADS / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int inc = v;
   for (int o = 1; o < 32; o <<= 1) {
     const int u = __shfl_up_sync(0xffffffffu, inc, o);
     if (lane >= o) inc += u;
   }
+  __syncthreads();  // s_warp may still be read for an earlier sum
   if (lane == 31) s_warp[warp] = inc;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int run = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-      const int x = s_warp[w];
-      s_warp[w] = run;
-      run += x;
-    }
-    *total = run;
+  int base = 0, all = 0;
+#pragma unroll
+  for (int w = 0; w < SCAN_THREADS / 32; ++w) {
+    base += (w < warp) ? s_warp[w] : 0;
+    all += s_warp[w];
   }
-  __syncthreads();
-  return s_warp[warp] + inc - v;
+  *total = all;
+  return base + inc - v;
 }
 
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_sums(const int* hist, int n, int* bsum) {
-  __shared__ int s_warp[SCAN_THREADS / 32];
-  __shared__ int s_total;
   const int base = blockIdx.x * SCAN_BLOCK;
-  int v = 0;
-  for (int e = threadIdx.x; e < SCAN_BLOCK; e += blockDim.x)
+  int v = 0, total;
+  for (int e = threadIdx.x; e < SCAN_BLOCK; e += SCAN_THREADS)
     if (base + e < n) v += hist[base + e];
-  block_exclusive_sum(v, s_warp, &s_total);
-  if (threadIdx.x == 0) bsum[blockIdx.x] = s_total;
+  block_exclusive_sum(v, &total);
+  if (threadIdx.x == 0) bsum[blockIdx.x] = total;
 }
 
-// start[i] = boff[block] + exclusive sum inside the block; start[n] = total
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_apply(const int* hist, int n, const int* boff, int* start) {
-  __shared__ int s_warp[SCAN_THREADS / 32];
-  __shared__ int s_total;
-  const int base = blockIdx.x * SCAN_BLOCK + threadIdx.x * SCAN_ITEMS;
-  int v[SCAN_ITEMS];
-  int sum = 0;
+// Block blk of the scan; before[0..nbefore) adds up to its first value.
+__device__ __forceinline__ void d_scan(const int* hist, int n, const int* before, int nbefore, int blk, int* start,
+                                       int* cursor) {
+  int v = 0, first, total;
+  for (int e = threadIdx.x; e < nbefore; e += SCAN_THREADS) v += before[e];
+  block_exclusive_sum(v, &first);
+  const int base = blk * SCAN_BLOCK + threadIdx.x * SCAN_ITEMS;
+  int h[SCAN_ITEMS], sum = 0;
 #pragma unroll
   for (int k = 0; k < SCAN_ITEMS; ++k) {
-    v[k] = (base + k < n) ? hist[base + k] : 0;
-    sum += v[k];
+    h[k] = (base + k < n) ? hist[base + k] : 0;
+    sum += h[k];
   }
-  int run = boff[blockIdx.x] + block_exclusive_sum(sum, s_warp, &s_total);
+  int run = first + block_exclusive_sum(sum, &total);
 #pragma unroll
   for (int k = 0; k < SCAN_ITEMS; ++k) {
-    if (base + k < n) start[base + k] = run;
-    run += v[k];
+    if (base + k < n) {
+      start[base + k] = run;
+      cursor[base + k] = run;
+    }
+    run += h[k];
     if (base + k == n - 1) start[n] = run;
   }
+}
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan(const int* hist, int n, const int* bsum, int* start, int* cursor) {
+  if (bsum) d_scan(hist, n, bsum, blockIdx.x, blockIdx.x, start, cursor);
+  else d_scan(hist, n, hist, blockIdx.x * SCAN_BLOCK, blockIdx.x, start, cursor);
 }
 
 // hist has nkeys+1 bins (the last one: removed particles).  scan_tmp holds
@@ -190,20 +175,13 @@ int bin_finish(const int* key, long long np, const TileGeo& t, const int* hist, 
                int* scan_tmp, cudaStream_t st, int sms) {
   const int n = t.nkeys + 1;
   const int nb = (n + SCAN_BLOCK - 1) / SCAN_BLOCK;
-  if (nb <= 1) {
-    k_scan_int<<<1, 1024, 0, st>>>(hist, n, start);
-  } else {
-    int* bsum = scan_tmp;
-    int* boff = scan_tmp + nb + 1;
-    k_scan_sums<<<nb, SCAN_THREADS, 0, st>>>(hist, n, bsum);
-    k_scan_int<<<1, 1024, 0, st>>>(bsum, nb, boff);
-    k_scan_apply<<<nb, SCAN_THREADS, 0, st>>>(hist, n, boff, start);
-  }
-  cudaMemsetAsync(cursor, 0, sizeof(int) * n, st);
-  if (np > 0) k_perm_scatter<<<grid_for(np, 256, sms, 16), 256, 0, st>>>(key, np, start, cursor, perm);
-  return (nb <= 1 ? 1 : 3) + (np > 0 ? 1 : 0);
+  const bool one = n <= SCAN_ONE;
+  if (!one) k_scan_sums<<<nb, SCAN_THREADS, 0, st>>>(hist, n, scan_tmp);
+  k_scan<<<nb, SCAN_THREADS, 0, st>>>(hist, n, one ? nullptr : scan_tmp, start, cursor);
+  if (np > 0) k_perm_scatter<<<grid_for(np, 256, sms, 16), 256, 0, st>>>(key, np, cursor, perm);
+  return (one ? 1 : 2) + (np > 0 ? 1 : 0);
 }
-int bin_scan_tmp_ints(const TileGeo& t) { return 2 * ((t.nkeys + 1) / SCAN_BLOCK + 3); }
+int bin_scan_tmp_ints(const TileGeo& t) { return (t.nkeys + 1) / SCAN_BLOCK + 1; }
 
 // ---- compaction along the permutation (physical reorder by tile) --------
 struct PermAlive {
@@ -288,20 +266,22 @@ long long perm_compact32(const int* perm, long long nalive, const Part32View& sr
 }
 
 
-// ---- multi-instance binning: scan (one block per instance), scatter ------
+// ---- multi-instance binning: scan, scatter (a row of blocks per instance) --
 namespace {
-__global__ void km_scan(const MultiInst* __restrict__ d) {
-  const MultiInst& m = d[blockIdx.x];
-  d_scan_int(m.ta.hist, m.ta.t.nkeys + 1, const_cast<int*>(m.ta.tstart));
+__global__ void __launch_bounds__(SCAN_THREADS) km_scan(const MultiInst* __restrict__ d) {
+  const MultiInst& m = d[blockIdx.y];
+  const int n = m.ta.t.nkeys + 1;
+  if ((int)blockIdx.x * SCAN_BLOCK >= n) return;
+  d_scan(m.ta.hist, n, m.ta.hist, blockIdx.x * SCAN_BLOCK, blockIdx.x, const_cast<int*>(m.ta.tstart), m.cursor);
 }
 __global__ void km_scatter(const MultiInst* __restrict__ d) {
   const MultiInst& m = d[blockIdx.y];
-  d_perm_scatter(m.ta.key, m.np, m.ta.tstart, m.cursor, const_cast<int*>(m.ta.perm), blockIdx.x, gridDim.x);
+  d_perm_scatter(m.ta.key, m.np, m.cursor, const_cast<int*>(m.ta.perm), blockIdx.x, gridDim.x);
 }
 }  // namespace
 
 void multi_bin32(const MultiInst* d, const MultiPlan& pl, cudaStream_t st, int* launches) {
-  km_scan<<<pl.n, 1024, 0, st>>>(d);
+  km_scan<<<dim3((pl.max_keys + SCAN_BLOCK) / SCAN_BLOCK, pl.n), SCAN_THREADS, 0, st>>>(d);
   km_scatter<<<dim3(pl.gx_parts, pl.n), 256, 0, st>>>(d);
   *launches += 2;
 }

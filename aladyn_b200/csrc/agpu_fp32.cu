@@ -16,8 +16,7 @@ namespace agpu {
 
 void field_bd32(const Dev32& d, cudaStream_t st, int sms) { field_bd_t<float>(d.ebf, d.g, st, sms); }
 void jfold32(const Dev32& d, cudaStream_t st, int sms) {
-  jfold_t<float>(d.jhi, d.g, st, sms);
-  jfold_t<float>(d.jlo, d.g, st, sms);
+  jfold_t<float>(d.jhi, d.jlo, d.g, st, sms);
 }
 void yee32(const Dev32& d, const YeeC& c, cudaStream_t st, int sms) { yee_t<float>(d.ebf, d.jhi, d.jlo, d.g, c, st, sms); }
 void yee32_fused(const float* fin, float* fout, const float* jhi, const float* jlo, const Geo& g, const YeeC& c,
@@ -433,7 +432,6 @@ __global__ void km_pre(const MultiInst* __restrict__ d) {
   }
   const int nt = m.ta.t.nkeys;
   GRID_STRIDE(b, (long long)nt + 1) {
-    m.cursor[b] = 0;
     if (b == nt) {
       const int alive = m.ta.tstart[nt];
       m.ta.hist[b] = (int)(m.np - alive);  // the records already dead
@@ -444,30 +442,11 @@ __global__ void km_pre(const MultiInst* __restrict__ d) {
       m.ta.hist[b] = 0;
     }
   }
-  d_field_bd_x<float>(m.ebf, g, g.nf, bid_, nb_);
+  d_field_bd<float>(m.ebf, g, g.nf, bid_, nb_);
 }
-__global__ void km_bd_y(const MultiInst* __restrict__ d) {
+__global__ void km_fold(const MultiInst* __restrict__ d) {
   const MultiInst& m = d[blockIdx.y];
-  d_field_bd_y<float>(m.ebf, m.ta.g, m.ta.g.nf, blockIdx.x, gridDim.x);
-}
-__global__ void km_bd_z(const MultiInst* __restrict__ d) {
-  const MultiInst& m = d[blockIdx.y];
-  d_field_bd_z<float>(m.ebf, m.ta.g, m.ta.g.nf, blockIdx.x, gridDim.x);
-}
-__global__ void km_fold_x(const MultiInst* __restrict__ d) {
-  const MultiInst& m = d[blockIdx.y];
-  d_jfold_x<float>(m.ta.jhi, m.ta.g, blockIdx.x, gridDim.x);
-  d_jfold_x<float>(m.ta.jlo, m.ta.g, blockIdx.x, gridDim.x);
-}
-__global__ void km_fold_y(const MultiInst* __restrict__ d) {
-  const MultiInst& m = d[blockIdx.y];
-  d_jfold_y<float>(m.ta.jhi, m.ta.g, blockIdx.x, gridDim.x);
-  d_jfold_y<float>(m.ta.jlo, m.ta.g, blockIdx.x, gridDim.x);
-}
-__global__ void km_fold_z(const MultiInst* __restrict__ d) {
-  const MultiInst& m = d[blockIdx.y];
-  d_jfold_z<float>(m.ta.jhi, m.ta.g, blockIdx.x, gridDim.x);
-  d_jfold_z<float>(m.ta.jlo, m.ta.g, blockIdx.x, gridDim.x);
+  d_jfold<float>(m.ta.jhi, m.ta.jlo, m.ta.g, blockIdx.x, gridDim.x);
 }
 __global__ void km_ef_bds(const MultiInst* __restrict__ d, int full_dt) {
   const MultiInst& m = d[blockIdx.y];
@@ -477,15 +456,42 @@ __global__ void km_bf_bds(const MultiInst* __restrict__ d) {
   const MultiInst& m = d[blockIdx.y];
   d_bf_bds<float>(m.ebf, m.ta.g, m.yc, m.yc.dt, blockIdx.x, gridDim.x);
 }
-template <int NDIM>
-__global__ void __launch_bounds__(256) km_rote(const MultiInst* __restrict__ d) {
+// The sweeps: the instance's blocks take its x-rows in turn, the threads run
+// along x.  ROTB: rotb_at, else rote_at.  The descriptor is copied: read
+// through the global pointer it would be reloaded after every store.
+template <int NDIM, bool BDS, bool ROTB>
+__global__ void __launch_bounds__(256) km_sweep(const MultiInst* __restrict__ d, int full_dt) {
   const MultiInst& m = d[blockIdx.y];
-  d_rote<float, NDIM>(m.ebf, m.ta.g, m.yc, 0.5 * m.yc.dt, blockIdx.x, gridDim.x);
+  const Geo g = m.ta.g;
+  const YeeC c = m.yc;
+  float* ebf = m.ebf;
+  const float *jhi = m.ta.jhi, *jlo = m.ta.jlo;
+  const int ny = g.jy2 - g.jy1 + 1, rows = ny * (g.kz2 - g.kz1 + 1);
+  for (int r = blockIdx.x; r < rows; r += gridDim.x) {
+    const int j = g.jy1 + r % ny, k = g.kz1 + r / ny;
+    for (int i = g.ix1 + threadIdx.x; i <= g.ix2; i += blockDim.x) {
+      if (ROTB) rotb_at<float, NDIM, BDS, !BDS>(ebf, jhi, jlo, g, c, c.dt, i, j, k);
+      else rote_at<float, NDIM, BDS, !BDS>(ebf, g, c, 0.5 * c.dt, full_dt ? c.dt : 0.0, i, j, k);
+    }
+  }
 }
 template <int NDIM>
-__global__ void __launch_bounds__(256) km_rotb_j(const MultiInst* __restrict__ d) {
-  const MultiInst& m = d[blockIdx.y];
-  d_rotb_j<float, NDIM>(m.ebf, m.ta.jhi, m.ta.jlo, m.ta.g, m.yc, m.yc.dt, blockIdx.x, gridDim.x);
+void multi_yee(const MultiInst* d, const MultiPlan& pl, cudaStream_t st, int* launches) {
+  const dim3 gf(pl.gx_faces, pl.n), gc(pl.gx_cells, pl.n);
+  if (pl.bds) {
+    km_sweep<NDIM, true, false><<<gc, 256, 0, st>>>(d, 0);
+    km_sweep<NDIM, true, true><<<gc, 256, 0, st>>>(d, 1);
+    km_sweep<NDIM, true, false><<<gc, 256, 0, st>>>(d, 1);
+    *launches += 3;
+    return;
+  }
+  km_ef_bds<<<gf, 256, 0, st>>>(d, 0);
+  km_sweep<NDIM, false, false><<<gc, 256, 0, st>>>(d, 0);
+  km_bf_bds<<<gf, 256, 0, st>>>(d);
+  km_sweep<NDIM, false, true><<<gc, 256, 0, st>>>(d, 1);
+  km_ef_bds<<<gf, 256, 0, st>>>(d, 1);
+  km_sweep<NDIM, false, false><<<gc, 256, 0, st>>>(d, 1);
+  *launches += 6;
 }
 
 }  // namespace
@@ -494,32 +500,13 @@ void multi_pre32(const MultiInst* d, const MultiPlan& pl, cudaStream_t st, int* 
   km_pre<<<dim3(pl.gx_cells, pl.n), 256, 0, st>>>(d);
   *launches += 1;
 }
-void multi_field_bd32(const MultiInst* d, const MultiPlan& pl, cudaStream_t st, int* launches) {
-  km_bd_y<<<dim3(pl.gx_faces, pl.n), 256, 0, st>>>(d);
-  *launches += 1;
-  if (pl.ndim == 3) {
-    km_bd_z<<<dim3(pl.gx_faces, pl.n), 256, 0, st>>>(d);
-    *launches += 1;
-  }
-}
 // the order of yee_t (curr_and_fields_util.f90:176-260): ef_bds(0), rote(dt/2),
 // bf_bds(dt), rotb + current(dt), ef_bds(dt), rote(dt/2)
 void multi_fields32(const MultiInst* d, const MultiPlan& pl, cudaStream_t st, int* launches) {
-  km_fold_x<<<dim3(pl.gx_faces, pl.n), 256, 0, st>>>(d);
-  km_fold_y<<<dim3(pl.gx_faces, pl.n), 256, 0, st>>>(d);
-  *launches += 2;
-  if (pl.ndim == 3) {
-    km_fold_z<<<dim3(pl.gx_faces, pl.n), 256, 0, st>>>(d);
-    *launches += 1;
-  }
-  const dim3 gf(pl.gx_faces, pl.n), gc(pl.gx_cells, pl.n);
-  km_ef_bds<<<gf, 256, 0, st>>>(d, 0);
-  if (pl.ndim == 3) km_rote<3><<<gc, 256, 0, st>>>(d); else km_rote<2><<<gc, 256, 0, st>>>(d);
-  km_bf_bds<<<gf, 256, 0, st>>>(d);
-  if (pl.ndim == 3) km_rotb_j<3><<<gc, 256, 0, st>>>(d); else km_rotb_j<2><<<gc, 256, 0, st>>>(d);
-  km_ef_bds<<<gf, 256, 0, st>>>(d, 1);
-  if (pl.ndim == 3) km_rote<3><<<gc, 256, 0, st>>>(d); else km_rote<2><<<gc, 256, 0, st>>>(d);
-  *launches += 6;
+  km_fold<<<dim3(pl.gx_faces, pl.n), 256, 0, st>>>(d);
+  *launches += 1;
+  if (pl.ndim == 3) multi_yee<3>(d, pl, st, launches);
+  else multi_yee<2>(d, pl, st, launches);
 }
 
 }  // namespace agpu

@@ -514,7 +514,7 @@ void push_deposit64(const PushArgs64& a, cudaStream_t st, int sms, bool serial) 
   }
 }
 
-void jfold64(const Dev64& d, cudaStream_t st, int sms) { jfold_t<double>(d.jc, d.g, st, sms); }
+void jfold64(const Dev64& d, cudaStream_t st, int sms) { jfold_t<double>(d.jc, (double*)nullptr, d.g, st, sms); }
 
 void yee64(const Dev64& d, const YeeC& c, cudaStream_t st, int sms, const XAdv* xa, YeeHook* hk) {
   yee_t<double>(d.ebf, d.jc, (const double*)nullptr, d.g, c, st, sms, xa, hk);

@@ -22,6 +22,10 @@ struct YeeC {
   double by3 = 1.0, ty4 = 1.0, bz3 = 1.0, tz4 = 1.0;
 };
 
+// Launches of one Yee step without advection substeps; separate: something
+// runs between its boundary and interior sweeps.
+inline int yee_launches(const YeeC& c, bool separate) { return (!separate && c.se2 == 0.0) ? 3 : 6; }
+
 // One stretched transverse axis (map2dy_part_sind / map2dz_part_sind,
 // src/grid/stretched_grid.f90:45-143): a particle coordinate in cells of the
 // uniform computational grid (node index - 1 of the integer nodes).

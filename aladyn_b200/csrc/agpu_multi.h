@@ -17,7 +17,7 @@ struct MultiInst {
   TileArgs32 ta;               // geometry, fields (read), currents, particles, binning arrays
   float* ebf;                  // fields (written by the field phases)
   YeeC yc;
-  int* cursor;                 // scatter cursors (nkeys + 1)
+  int* cursor;                 // scatter cursors (nkeys + 1), set by the scan
   unsigned long long* pushed;  // the instance's device push counter
   unsigned long long* removed;
   double* fmax;
@@ -31,13 +31,13 @@ struct MultiPlan {
   int gx_cells;       // blocks per instance for cell-wide phases
   int gx_faces;       // blocks per instance for face-wide phases
   int gx_parts;       // blocks per instance for particle-wide phases
+  int max_keys;       // most binning keys of an instance
+  int bds;            // every instance has se2 = 0: boundary ghosts in the Yee sweeps
 };
 
-// pre: currents and cursors zeroed, next histogram seeded, push counter and
-// step counters; then the x-face field extrapolation (field_xyzbd, x).
+// pre: currents zeroed, next histogram seeded, push counter and
+// step counters; the field extrapolation (field_xyzbd).
 void multi_pre32(const MultiInst* d, const MultiPlan& pl, cudaStream_t st, int* launches);
-// y (and z) face extrapolation
-void multi_field_bd32(const MultiInst* d, const MultiPlan& pl, cudaStream_t st, int* launches);
 // gather + push + deposit of every tile of every instance
 void multi_tile32(const MultiInst* d, const int* tile_off, const MultiPlan& pl, cudaStream_t st, int* launches);
 // scan of the next histogram and the permutation scatter

@@ -926,11 +926,10 @@ size_t tile32_smem(int ndim) { return sizeof(float) * (size_t)((ndim == 3) ? CT<
 
 int tile32_list_cap(int ndim) { return (ndim == 3) ? CT<3>::LIST_CAP : CT<2>::LIST_CAP; }
 
-// Returns the kernels launched (the work-list counters are reset here).
+// Returns the kernels launched (hist_reset has cleared the work-list counters).
 int tile_push32(const TileArgs32& a, cudaStream_t st, int sms) {
   if (a.t.ntiles <= 0) return 0;
   const size_t sm = tile32_smem(a.g.ndim);
-  if (a.work) cudaMemsetAsync(a.work_n, 0, 2 * sizeof(unsigned int), st);
   if (a.g.ndim == 3) {
     auto k = k32_tile<3>;
     auto k2 = k32_tile_more<3>;

@@ -4,6 +4,8 @@
 // compiled without FMA contraction so the statement order of the reference
 // is kept bit for bit) and agpu_fp32.cu (T = float).
 #pragma once
+#include <type_traits>
+
 #include "agpu_common.cuh"
 #include "agpu_kernels.h"
 
@@ -17,142 +19,152 @@ namespace agpu {
   for (long long t = bid_ * (long long)blockDim.x + threadIdx.x; t < (total); t += nb_ * (long long)blockDim.x)
 
 // ---- A1: field_xyzbd (src/parallel/mpi_field_interface.f90:53-198) --------
+// One ghost layer by linear extrapolation along x, then y over the widened x
+// range, then z over the widened x and y ranges.  A ghost of a later axis is
+// formed from the earlier axes' extrapolations of the interior (the same
+// operations on the same values), so one sweep reads interior nodes only
+// and writes every ghost: one launch instead of a dependent one per axis
+// (4 us each on the small grids, where a launch costs more than its work).
 template <typename T>
-__device__ __forceinline__ void d_field_bd_x(T* ebf, Geo g, int nc, long long bid_, long long nb_) {
-  int ny = g.jy2 - g.jy1 + 1, nz = g.kz2 - g.kz1 + 1;
-  long long total = (long long)ny * nz * nc;
-  GRID_STRIDE(t, total) {
-    int iy = g.jy1 + (int)(t % ny);
-    int iz = g.kz1 + (int)((t / ny) % nz);
-    int ik = (int)(t / ((long long)ny * nz));
+__device__ __forceinline__ T bd_x(const T* f, const Geo& g, int i, int j, int k) {
+  if (i < g.ix1) return (T)2. * f[goff(g, g.ix1, j, k)] - f[goff(g, g.ix1 + 1, j, k)];
+  if (i > g.ix2) return (T)2. * f[goff(g, g.ix2, j, k)] - f[goff(g, g.ix2 - 1, j, k)];
+  return f[goff(g, i, j, k)];
+}
+template <typename T>
+__device__ __forceinline__ T bd_y(const T* f, const Geo& g, int i, int j, int k) {
+  if (j < g.jy1) return (T)2. * bd_x(f, g, i, g.jy1, k) - bd_x(f, g, i, g.jy1 + 1, k);
+  if (j > g.jy2) return (T)2. * bd_x(f, g, i, g.jy2, k) - bd_x(f, g, i, g.jy2 - 1, k);
+  return bd_x(f, g, i, j, k);
+}
+template <typename T>
+__device__ __forceinline__ T bd_z(const T* f, const Geo& g, int i, int j, int k) {
+  if (k < g.kz1) return (T)2. * bd_y(f, g, i, j, g.kz1) - bd_y(f, g, i, j, g.kz1 + 1);
+  return (T)2. * bd_y(f, g, i, j, g.kz2) - bd_y(f, g, i, j, g.kz2 - 1);
+}
+// ghost nodes of one component: two x faces, two y faces, two z faces (3D)
+AGPU_HD int bd_nodes(const Geo& g) {
+  const int nx = g.ix2 - g.ix1 + 1, ny = g.jy2 - g.jy1 + 1, nz = g.kz2 - g.kz1 + 1;
+  return 2 * (ny * nz + (nx + 2) * nz + (g.ndim == 3 ? (nx + 2) * (ny + 2) : 0));
+}
+template <typename T>
+__device__ __forceinline__ void d_field_bd(T* ebf, const Geo& g, int nc, long long bid_, long long nb_) {
+  const int nxe = g.ix2 - g.ix1 + 3, nye = g.jy2 - g.jy1 + 3, ny = nye - 2, nz = g.kz2 - g.kz1 + 1;
+  const int n = bd_nodes(g), fx = 2 * ny * nz, fy = 2 * nxe * nz;
+  GRID_STRIDE(t, (long long)n * nc) {
+    const int ik = (int)(t / n);
+    int r = (int)(t - (long long)ik * n);
     T* f = ebf + g.ncell * ik;
-    f[goff(g, g.ix1 - 1, iy, iz)] = (T)2. * f[goff(g, g.ix1, iy, iz)] - f[goff(g, g.ix1 + 1, iy, iz)];
-    f[goff(g, g.ix2 + 1, iy, iz)] = (T)2. * f[goff(g, g.ix2, iy, iz)] - f[goff(g, g.ix2 - 1, iy, iz)];
+    int i, j, k;
+    T v;
+    if (r < fx) {
+      const int hi = r >= fx / 2;
+      r -= hi * (fx / 2);
+      i = hi ? g.ix2 + 1 : g.ix1 - 1;
+      j = g.jy1 + r % ny;
+      k = g.kz1 + r / ny;
+      v = bd_x(f, g, i, j, k);
+    } else if (r < fx + fy) {
+      r -= fx;
+      const int hi = r >= fy / 2;
+      r -= hi * (fy / 2);
+      i = g.ix1 - 1 + r % nxe;
+      j = hi ? g.jy2 + 1 : g.jy1 - 1;
+      k = g.kz1 + r / nxe;
+      v = bd_y(f, g, i, j, k);
+    } else {
+      r -= fx + fy;
+      const int hi = r >= nxe * nye;
+      r -= hi * (nxe * nye);
+      i = g.ix1 - 1 + r % nxe;
+      j = g.jy1 - 1 + r / nxe;
+      k = hi ? g.kz2 + 1 : g.kz1 - 1;
+      v = bd_z(f, g, i, j, k);
+    }
+    f[goff(g, i, j, k)] = v;
   }
 }
 template <typename T>
-__global__ void k_field_bd_x(T* ebf, Geo g, int nc) {
-  d_field_bd_x<T>(ebf, g, nc, blockIdx.x, gridDim.x);
-}
-template <typename T>
-__device__ __forceinline__ void d_field_bd_y(T* ebf, Geo g, int nc, long long bid_, long long nb_) {
-  int nxe = g.ix2 - g.ix1 + 3, nz = g.kz2 - g.kz1 + 1;
-  long long total = (long long)nxe * nz * nc;
-  GRID_STRIDE(t, total) {
-    int ix = g.ix1 - 1 + (int)(t % nxe);
-    int iz = g.kz1 + (int)((t / nxe) % nz);
-    int ik = (int)(t / ((long long)nxe * nz));
-    T* f = ebf + g.ncell * ik;
-    f[goff(g, ix, g.jy1 - 1, iz)] = (T)2. * f[goff(g, ix, g.jy1, iz)] - f[goff(g, ix, g.jy1 + 1, iz)];
-    f[goff(g, ix, g.jy2 + 1, iz)] = (T)2. * f[goff(g, ix, g.jy2, iz)] - f[goff(g, ix, g.jy2 - 1, iz)];
-  }
-}
-template <typename T>
-__global__ void k_field_bd_y(T* ebf, Geo g, int nc) {
-  d_field_bd_y<T>(ebf, g, nc, blockIdx.x, gridDim.x);
-}
-template <typename T>
-__device__ __forceinline__ void d_field_bd_z(T* ebf, Geo g, int nc, long long bid_, long long nb_) {
-  int nxe = g.ix2 - g.ix1 + 3, nye = g.jy2 - g.jy1 + 3;
-  long long total = (long long)nxe * nye * nc;
-  GRID_STRIDE(t, total) {
-    int ix = g.ix1 - 1 + (int)(t % nxe);
-    int iy = g.jy1 - 1 + (int)((t / nxe) % nye);
-    int ik = (int)(t / ((long long)nxe * nye));
-    T* f = ebf + g.ncell * ik;
-    f[goff(g, ix, iy, g.kz1 - 1)] = (T)2 * f[goff(g, ix, iy, g.kz1)] - f[goff(g, ix, iy, g.kz1 + 1)];
-    f[goff(g, ix, iy, g.kz2 + 1)] = (T)2 * f[goff(g, ix, iy, g.kz2)] - f[goff(g, ix, iy, g.kz2 - 1)];
-  }
-}
-template <typename T>
-__global__ void k_field_bd_z(T* ebf, Geo g, int nc) {
-  d_field_bd_z<T>(ebf, g, nc, blockIdx.x, gridDim.x);
+__global__ void k_field_bd(T* ebf, Geo g, int nc) {
+  d_field_bd<T>(ebf, g, nc, blockIdx.x, gridDim.x);
 }
 template <typename T>
 void field_bd_t(T* ebf, const Geo& g, cudaStream_t st, int sms) {
-  int nc = g.nf;
-  k_field_bd_x<T><<<grid_for((long long)(g.jy2 - g.jy1 + 1) * (g.kz2 - g.kz1 + 1) * nc, 256, sms), 256, 0, st>>>(ebf, g, nc);
-  k_field_bd_y<T><<<grid_for((long long)(g.ix2 - g.ix1 + 3) * (g.kz2 - g.kz1 + 1) * nc, 256, sms), 256, 0, st>>>(ebf, g, nc);
-  if (g.ndim == 3)
-    k_field_bd_z<T><<<grid_for((long long)(g.ix2 - g.ix1 + 3) * (g.jy2 - g.jy1 + 3) * nc, 256, sms), 256, 0, st>>>(ebf, g, nc);
+  k_field_bd<T><<<grid_for((long long)bd_nodes(g) * g.nf, 256, sms), 256, 0, st>>>(ebf, g, g.nf);
 }
 
 // ---- A13: jc_xyzbd (src/parallel/mpi_curr_interface.f90:551-643) ----------
+// The ghost currents added to the faces' nodes and cleared, x, then y, then
+// z.  A node's ghosts along one axis lie on interior nodes of the others, so
+// no fold touches what another reads: one sweep over the boundary nodes adds
+// them in that order, for both parts of a two-float current.
+// boundary nodes of one component: the x faces, then what the y and z faces
+// have beyond them
+AGPU_HD int fold_nodes(const Geo& g) {
+  const int nx = g.ix2 - g.ix1 + 1, ny = g.jy2 - g.jy1 + 1, nz = g.kz2 - g.kz1 + 1;
+  return 2 * (ny * nz + (nx - 2) * nz + (g.ndim == 3 ? (nx - 2) * (ny - 2) : 0));
+}
 template <typename T>
-__device__ __forceinline__ void d_jfold_x(T* jc, Geo g, long long bid_, long long nb_) {
-  int ny = g.jy2 - g.jy1 + 1, nz = g.kz2 - g.kz1 + 1;
-  long long total = (long long)ny * nz * g.nc;
-  GRID_STRIDE(t, total) {
-    int j = g.jy1 + (int)(t % ny);
-    int k = g.kz1 + (int)((t / ny) % nz);
-    int ik = (int)(t / ((long long)ny * nz));
-    T* c = jc + g.ncell * ik;
-    long long a = goff(g, g.ix1, j, k);
-    c[a] = c[a] + c[a - 1];
-    c[a - 1] = (T)0;
-    long long b = goff(g, g.ix2, j, k);
-    c[b] = c[b] + c[b + 1] + c[b + 2];
-    c[b + 1] = (T)0;
-    c[b + 2] = (T)0;
+__device__ __forceinline__ void d_jfold(T* j0, T* j1, const Geo& g, long long bid_, long long nb_) {
+  const int nx = g.ix2 - g.ix1 + 1, ny = g.jy2 - g.jy1 + 1, nz = g.kz2 - g.kz1 + 1;
+  const int n = fold_nodes(g), fx = 2 * ny * nz, fy = 2 * (nx - 2) * nz;
+  const long long sy = g.n1p, sz = (long long)g.n1p * g.n2p;
+  GRID_STRIDE(t, (long long)n * g.nc * (j1 ? 2 : 1)) {
+    const int q = (int)(t / n);
+    int r = (int)(t - (long long)q * n);
+    int i, j, k;
+    if (r < fx) {
+      const int hi = r >= fx / 2;
+      r -= hi * (fx / 2);
+      i = hi ? g.ix2 : g.ix1;
+      j = g.jy1 + r % ny;
+      k = g.kz1 + r / ny;
+    } else if (r < fx + fy) {
+      r -= fx;
+      const int hi = r >= fy / 2;
+      r -= hi * (fy / 2);
+      i = g.ix1 + 1 + r % (nx - 2);
+      j = hi ? g.jy2 : g.jy1;
+      k = g.kz1 + r / (nx - 2);
+    } else {
+      r -= fx + fy;
+      const int m = (nx - 2) * (ny - 2), hi = r >= m;
+      r -= hi * m;
+      i = g.ix1 + 1 + r % (nx - 2);
+      j = g.jy1 + 1 + r / (nx - 2);
+      k = hi ? g.kz2 : g.kz1;
+    }
+    T* c = (q < g.nc ? j0 + g.ncell * q : j1 + g.ncell * (q - g.nc)) + goff(g, i, j, k);
+    T v = *c;
+    // the nearer, then the farther ghost node along one direction
+    auto two = [&](long long d) {
+      v = v + c[d] + c[2 * d];
+      c[d] = (T)0;
+      c[2 * d] = (T)0;
+    };
+    auto one = [&](long long d) {
+      v = v + c[d];
+      c[d] = (T)0;
+    };
+    if (i == g.ix1) one(-1);
+    if (i == g.ix2) two(1);
+    if (j == g.jy1) two(-sy);
+    if (j == g.jy2) two(sy);
+    if (g.ndim == 3) {
+      if (k == g.kz1) one(-sz);
+      if (k == g.kz2) two(sz);
+    }
+    *c = v;
   }
 }
 template <typename T>
-__global__ void k_jfold_x(T* jc, Geo g) {
-  d_jfold_x<T>(jc, g, blockIdx.x, gridDim.x);
+__global__ void k_jfold(T* j0, T* j1, Geo g) {
+  d_jfold<T>(j0, j1, g, blockIdx.x, gridDim.x);
 }
+// j1: the compensation part of a two-float current, or null
 template <typename T>
-__device__ __forceinline__ void d_jfold_y(T* jc, Geo g, long long bid_, long long nb_) {
-  int nx = g.ix2 - g.ix1 + 1, nz = g.kz2 - g.kz1 + 1;
-  long long total = (long long)nx * nz * g.nc;
-  long long sy = g.n1p;
-  GRID_STRIDE(t, total) {
-    int ix = g.ix1 + (int)(t % nx);
-    int iz = g.kz1 + (int)((t / nx) % nz);
-    int ik = (int)(t / ((long long)nx * nz));
-    T* c = jc + g.ncell * ik;
-    long long a = goff(g, ix, g.jy1, iz);
-    c[a] = c[a] + c[a - sy] + c[a - 2 * sy];
-    c[a - 2 * sy] = (T)0;
-    c[a - sy] = (T)0;
-    long long b = goff(g, ix, g.jy2, iz);
-    c[b] = c[b] + c[b + sy] + c[b + 2 * sy];
-    c[b + sy] = (T)0;
-    c[b + 2 * sy] = (T)0;
-  }
-}
-template <typename T>
-__global__ void k_jfold_y(T* jc, Geo g) {
-  d_jfold_y<T>(jc, g, blockIdx.x, gridDim.x);
-}
-template <typename T>
-__device__ __forceinline__ void d_jfold_z(T* jc, Geo g, long long bid_, long long nb_) {
-  int nx = g.ix2 - g.ix1 + 1, ny = g.jy2 - g.jy1 + 1;
-  long long total = (long long)nx * ny * g.nc;
-  long long sz = (long long)g.n1p * g.n2p;
-  GRID_STRIDE(t, total) {
-    int ix = g.ix1 + (int)(t % nx);
-    int iy = g.jy1 + (int)((t / nx) % ny);
-    int ik = (int)(t / ((long long)nx * ny));
-    T* c = jc + g.ncell * ik;
-    long long a = goff(g, ix, iy, g.kz1);
-    c[a] = c[a] + c[a - sz];
-    c[a - sz] = (T)0;
-    long long b = goff(g, ix, iy, g.kz2);
-    c[b] = c[b] + c[b + sz] + c[b + 2 * sz];
-    c[b + sz] = (T)0;
-    c[b + 2 * sz] = (T)0;
-  }
-}
-template <typename T>
-__global__ void k_jfold_z(T* jc, Geo g) {
-  d_jfold_z<T>(jc, g, blockIdx.x, gridDim.x);
-}
-template <typename T>
-void jfold_t(T* jc, const Geo& g, cudaStream_t st, int sms) {
-  k_jfold_x<T><<<grid_for((long long)(g.jy2 - g.jy1 + 1) * (g.kz2 - g.kz1 + 1) * g.nc, 256, sms), 256, 0, st>>>(jc, g);
-  k_jfold_y<T><<<grid_for((long long)(g.ix2 - g.ix1 + 1) * (g.kz2 - g.kz1 + 1) * g.nc, 256, sms), 256, 0, st>>>(jc, g);
-  if (g.ndim == 3)
-    k_jfold_z<T><<<grid_for((long long)(g.ix2 - g.ix1 + 1) * (g.jy2 - g.jy1 + 1) * g.nc, 256, sms), 256, 0, st>>>(jc, g);
+void jfold_t(T* j0, T* j1, const Geo& g, cudaStream_t st, int sms) {
+  k_jfold<T><<<grid_for((long long)fold_nodes(g) * g.nc * (j1 ? 2 : 1), 256, sms), 256, 0, st>>>(j0, j1, g);
 }
 
 // ---- A14: Yee (advance_lpf_fields, curr_and_fields_util.f90:176-260) ------
@@ -246,191 +258,186 @@ __global__ void k_bf_bds(T* ebf, Geo g, YeeC c, double dtl) {
   d_bf_bds<T>(ebf, g, c, dtl, blockIdx.x, gridDim.x);
 }
 
-// rote (grid_fields.f90:1405-1478): B -= dtf curl E, interior.
-template <typename T, int NDIM>
-__device__ __forceinline__ void d_rote(T* ebf, Geo g, YeeC c, double dtf, long long bid_, long long nb_) {
-  int nx = g.ix2 - g.ix1 + 1, ny = g.jy2 - g.jy1 + 1, nz = g.kz2 - g.kz1 + 1;
-  long long total = (long long)nx * ny * nz;
-  double aphxd = dtf * c.dx_inv, aphyd = dtf * c.dy_inv, aphzd = dtf * c.dz_inv;
-  T aph1 = (T)(aphxd * c.se1), aph2 = (T)(aphxd * c.se2);
-  T sdhy = (T)(1.0 * aphyd), sdhz = (T)(1.0 * aphzd);
-  const T* E1 = ebf;
-  const T* E2 = ebf + g.ncell;
-  const T* E3 = ebf + 2 * g.ncell;
-  long long sy = g.n1p, sz = (long long)g.n1p * g.n2p;
-  GRID_STRIDE(t, total) {
-    int i = g.ix1 + (int)(t % nx);
-    int j = g.jy1 + (int)((t / nx) % ny);
-    int k = g.kz1 + (int)(t / ((long long)nx * ny));
-    long long o = goff(g, i, j, k);
-    if (NDIM == 2) {
-      T* Bz = ebf + 2 * g.ncell;
-      Bz[o] = Bz[o] - aph1 * (E2[o + 1] - E2[o]) + sdhy * (E1[o + sy] - E1[o]) - aph2 * (E2[o + 2] - E2[o - 1]);
+// rote (grid_fields.f90:1405-1478): B -= dtf curl E at node o = (i, j, k).
+// BDS: the right-face Mur ghosts of E (ef_bds with dtl), which this node's
+// differences read, depend on this node's fields alone, so the node forms and
+// stores them itself and no boundary sweep runs before this one.  Only with
+// the compact x difference (SE2 false: se2 = 0), whose stencil has no node
+// further out.
+template <typename T, int NDIM, bool BDS, bool SE2>
+__device__ __forceinline__ void rote_node(T* ebf, const Geo& g, const YeeC& c, long long o, int i, int j, int k, T aph1,
+                                          T aph2, T sdhy, T sdhz, double dtl) {
+  const long long sy = g.n1p, sz = (long long)g.n1p * g.n2p;
+  T* E1 = ebf;
+  T* E2 = ebf + g.ncell;
+  T* E3 = ebf + 2 * g.ncell;
+  T* Bx = ebf + 3 * g.ncell;
+  T* By = ebf + 4 * g.ncell;
+  T* Bz = ebf + (NDIM == 3 ? 5 : 2) * g.ncell;
+  const T e1 = E1[o], e2 = E2[o], e3 = (NDIM == 3) ? E3[o] : (T)0;
+  const T bz = Bz[o], bx = (NDIM == 3) ? Bx[o] : (T)0, by = (NDIM == 3) ? By[o] : (T)0;
+  T e2x, e3x = (T)0, e1y, e3y = (T)0, e1z = (T)0, e2z = (T)0;  // E one node up along x, y, z
+  const T one = (T)1., two = (T)2.;
+  if (BDS && i == g.ix2) {
+    const T aphx = (T)(1.0 * c.dx_inv * dtl);
+    E2[o + 1] = e2x = (two * bz - (one - aphx) * e2) / (one + aphx);
+    if (NDIM == 3) E3[o + 1] = e3x = -(two * by + (one - aphx) * e3) / (one + aphx);
+  } else {
+    e2x = E2[o + 1];
+    if (NDIM == 3) e3x = E3[o + 1];
+  }
+  if (BDS && j == g.jy2) {
+    const T aphy = (T)(c.ty4 * c.dy_inv * dtl);  // loc_yg(ny, 4) dy_inv dt
+    E1[o + sy] = e1y = -(two * bz + (one - aphy) * e1) / (one + aphy);
+    if (NDIM == 3) E3[o + sy] = e3y = (two * bx - (one - aphy) * e3) / (one + aphy);
+  } else {
+    e1y = E1[o + sy];
+    if (NDIM == 3) e3y = E3[o + sy];
+  }
+  if (NDIM == 3) {
+    if (BDS && k == g.kz2) {
+      const T aphz = (T)(c.tz4 * c.dz_inv * dtl);  // loc_zg(nz, 4) dz_inv dt
+      E1[o + sz] = e1z = (two * by - (one - aphz) * e1) / (one + aphz);
+      E2[o + sz] = e2z = -(two * bx + (one - aphz) * e2) / (one + aphz);
     } else {
-      T* Bx = ebf + 3 * g.ncell;
-      T* By = ebf + 4 * g.ncell;
-      T* Bz = ebf + 5 * g.ncell;
-      Bz[o] = Bz[o] - aph1 * (E2[o + 1] - E2[o]) + sdhy * (E1[o + sy] - E1[o]) - aph2 * (E2[o + 2] - E2[o - 1]);
-      Bx[o] = Bx[o] - sdhy * (E3[o + sy] - E3[o]) + sdhz * (E2[o + sz] - E2[o]);
-      By[o] = By[o] + aph1 * (E3[o + 1] - E3[o]) - sdhz * (E1[o + sz] - E1[o]) + aph2 * (E3[o + 2] - E3[o - 1]);
+      e1z = E1[o + sz];
+      e2z = E2[o + sz];
     }
   }
-}
-template <typename T, int NDIM>
-__global__ void __launch_bounds__(256) k_rote(T* ebf, Geo g, YeeC c, double dtf) {
-  d_rote<T, NDIM>(ebf, g, c, dtf, blockIdx.x, gridDim.x);
+  const T nz = bz - aph1 * (e2x - e2) + sdhy * (e1y - e1);
+  Bz[o] = SE2 ? nz - aph2 * (E2[o + 2] - E2[o - 1]) : nz;
+  if (NDIM == 3) {
+    Bx[o] = bx - sdhy * (e3y - e3) + sdhz * (e2z - e2);
+    const T ny = by + aph1 * (e3x - e3) - sdhz * (e1z - e1);
+    By[o] = SE2 ? ny + aph2 * (E3[o + 2] - E3[o - 1]) : ny;
+  }
 }
 
 // rotb (grid_fields.f90:1480-1552) + E -= ompe * (djc * J)
-// (curr_and_fields_util.f90:111-115, 227-231).  jlo (optional) holds the
-// compensation term of a two-float current.
-template <typename T, int NDIM>
-__device__ __forceinline__ void d_rotb_j(T* ebf, const T* jc, const T* jlo, Geo g, YeeC c, double dtf, long long bid_, long long nb_) {
-  int nx = g.ix2 - g.ix1 + 1, ny = g.jy2 - g.jy1 + 1, nz = g.kz2 - g.kz1 + 1;
-  long long total = (long long)nx * ny * nz;
-  double aphxd = dtf * c.dx_inv, aphyd = dtf * c.dy_inv, aphzd = dtf * c.dz_inv;
-  T aph1 = (T)(aphxd * c.se1), aph2 = (T)(aphxd * c.se2);
-  T sdy = (T)(1.0 * aphyd), sdz = (T)(aphzd * 1.0);
-  T ompe = (T)c.ompe, djc1 = (T)c.djc1, djc2 = (T)c.djc2, djc3 = (T)c.djc3;
+// (curr_and_fields_util.f90:111-115, 227-231) at node o.  jlo (optional)
+// holds the compensation term of a two-float current.  BDS: the left-face
+// Mur ghosts of B (bf_bds with dt) formed by the nodes that read them, as in
+// rote_node.
+template <typename T, int NDIM, bool BDS, bool SE2>
+__device__ __forceinline__ void rotb_node(T* ebf, const T* jc, const T* jlo, const Geo& g, const YeeC& c, long long o,
+                                          int i, int j, int k, T aph1, T aph2, T sdy, T sdz, double dtl) {
+  const long long sy = g.n1p, sz = (long long)g.n1p * g.n2p;
   T* E1 = ebf;
   T* E2 = ebf + g.ncell;
-  long long sy = g.n1p, sz = (long long)g.n1p * g.n2p;
-  GRID_STRIDE(t, total) {
-    int i = g.ix1 + (int)(t % nx);
-    int j = g.jy1 + (int)((t / nx) % ny);
-    int k = g.kz1 + (int)(t / ((long long)nx * ny));
-    long long o = goff(g, i, j, k);
-    T j1 = jc[o], j2 = jc[o + g.ncell];
-    if (jlo) {
-      j1 = j1 + jlo[o];
-      j2 = j2 + jlo[o + g.ncell];
-    }
-    if (NDIM == 2) {
-      const T* Bz = ebf + 2 * g.ncell;
-      T ex = E1[o] + sdy * (Bz[o] - Bz[o - sy]);
-      T ey = E2[o] - aph1 * (Bz[o] - Bz[o - 1]) - aph2 * (Bz[o + 1] - Bz[o - 2]);
-      E1[o] = ex - ompe * (djc1 * j1);
-      E2[o] = ey - ompe * (djc2 * j2);
-    } else {
-      T* E3 = ebf + 2 * g.ncell;
-      const T* Bx = ebf + 3 * g.ncell;
-      const T* By = ebf + 4 * g.ncell;
-      const T* Bz = ebf + 5 * g.ncell;
-      T j3 = jc[o + 2 * g.ncell];
-      if (jlo) j3 = j3 + jlo[o + 2 * g.ncell];
-      T ex = E1[o] + sdy * (Bz[o] - Bz[o - sy]);
-      T ey = E2[o] - aph1 * (Bz[o] - Bz[o - 1]) - aph2 * (Bz[o + 1] - Bz[o - 2]);
-      ex = ex - sdz * (By[o] - By[o - sz]);
-      ey = ey + sdz * (Bx[o] - Bx[o - sz]);
-      T ez = E3[o] + aph1 * (By[o] - By[o - 1]) - sdy * (Bx[o] - Bx[o - sy]) + aph2 * (By[o + 1] - By[o - 2]);
-      E1[o] = ex - ompe * (djc1 * j1);
-      E2[o] = ey - ompe * (djc2 * j2);
-      E3[o] = ez - ompe * (djc3 * j3);
-    }
-  }
-}
-template <typename T, int NDIM>
-__global__ void __launch_bounds__(256) k_rotb_j(T* ebf, const T* jc, const T* jlo, Geo g, YeeC c, double dtf) {
-  d_rotb_j<T, NDIM>(ebf, jc, jlo, g, c, dtf, blockIdx.x, gridDim.x);
-}
-
-// Single-instance forms of the two sweeps: one thread per node, blocks of
-// 128 x 2 nodes over (i, j) and one z plane per grid layer, so the node
-// indices come without the 64-bit divisions of the grid-stride bodies (which
-// serve the multi-instance kernels).  Every node's arithmetic is that of
-// d_rote / d_rotb_j, in the same order.  Measured on the 1024x256x256 grid:
-// the FP32 phase 2.42 -> 2.06 ms; marching each thread over several z planes
-// (carrying the z-neighbour loads) was slower.
-constexpr int YEE_BX = 128, YEE_BY = 2;
-
-template <typename T, int NDIM>
-__global__ void __launch_bounds__(YEE_BX* YEE_BY) k_rote_n(T* ebf, Geo g, YeeC c, double dtf) {
-  const int i = g.ix1 + blockIdx.x * YEE_BX + threadIdx.x;
-  const int j = g.jy1 + blockIdx.y * YEE_BY + threadIdx.y;
-  if (i > g.ix2 || j > g.jy2) return;
-  const double aphxd = dtf * c.dx_inv, aphyd = dtf * c.dy_inv, aphzd = dtf * c.dz_inv;
-  const T aph1 = (T)(aphxd * c.se1), aph2 = (T)(aphxd * c.se2);
-  // loc_yg(jj, 4) * aphy, loc_zg(kk, 4) * aphz (1 on a uniform axis)
-  const int kn = (NDIM == 3) ? g.kz1 + (int)blockIdx.z : 1;
-  const T sdhy = (T)((c.my4 ? c.my4[j - 2] : 1.0) * aphyd);
-  const T sdhz = (T)((c.mz4 && NDIM == 3 ? c.mz4[kn - 2] : 1.0) * aphzd);
-  const T* __restrict__ E1 = ebf;
-  const T* __restrict__ E2 = ebf + g.ncell;
-  const T* __restrict__ E3 = ebf + 2 * g.ncell;
-  const long long sy = g.n1p, sz = (long long)g.n1p * g.n2p;
-  if (NDIM == 2) {
-    const long long o = goff(g, i, j, 1);
-    T* Bz = ebf + 2 * g.ncell;
-    Bz[o] = Bz[o] - aph1 * (E2[o + 1] - E2[o]) + sdhy * (E1[o + sy] - E1[o]) - aph2 * (E2[o + 2] - E2[o - 1]);
-    return;
-  }
-  T* __restrict__ Bx = ebf + 3 * g.ncell;
-  T* __restrict__ By = ebf + 4 * g.ncell;
-  T* __restrict__ Bz = ebf + 5 * g.ncell;
-  const long long o = goff(g, i, j, kn);
-  Bz[o] = Bz[o] - aph1 * (E2[o + 1] - E2[o]) + sdhy * (E1[o + sy] - E1[o]) - aph2 * (E2[o + 2] - E2[o - 1]);
-  Bx[o] = Bx[o] - sdhy * (E3[o + sy] - E3[o]) + sdhz * (E2[o + sz] - E2[o]);
-  By[o] = By[o] + aph1 * (E3[o + 1] - E3[o]) - sdhz * (E1[o + sz] - E1[o]) + aph2 * (E3[o + 2] - E3[o - 1]);
-}
-
-template <typename T, int NDIM>
-__global__ void __launch_bounds__(YEE_BX* YEE_BY) k_rotb_j_n(T* ebf, const T* jc, const T* jlo, Geo g, YeeC c, double dtf) {
-  const int i = g.ix1 + blockIdx.x * YEE_BX + threadIdx.x;
-  const int j = g.jy1 + blockIdx.y * YEE_BY + threadIdx.y;
-  if (i > g.ix2 || j > g.jy2) return;
-  const double aphxd = dtf * c.dx_inv, aphyd = dtf * c.dy_inv, aphzd = dtf * c.dz_inv;
-  const T aph1 = (T)(aphxd * c.se1), aph2 = (T)(aphxd * c.se2);
-  // loc_yg(jj, 3) * aphy, aphz * loc_zg(kk, 3) (1 on a uniform axis)
-  const int kn = (NDIM == 3) ? g.kz1 + (int)blockIdx.z : 1;
-  const T sdy = (T)((c.my3 ? c.my3[j - 2] : 1.0) * aphyd);
-  const T sdz = (T)(aphzd * (c.mz3 && NDIM == 3 ? c.mz3[kn - 2] : 1.0));
+  T* E3 = ebf + 2 * g.ncell;
+  T* Bx = ebf + 3 * g.ncell;
+  T* By = ebf + 4 * g.ncell;
+  T* Bz = ebf + (NDIM == 3 ? 5 : 2) * g.ncell;
   const T ompe = (T)c.ompe, djc1 = (T)c.djc1, djc2 = (T)c.djc2, djc3 = (T)c.djc3;
-  T* __restrict__ E1 = ebf;
-  T* __restrict__ E2 = ebf + g.ncell;
-  const long long sy = g.n1p, sz = (long long)g.n1p * g.n2p;
-  const long long o = goff(g, i, j, kn);
-  T j1 = jc[o], j2 = jc[o + g.ncell];
+  T j1 = jc[o], j2 = jc[o + g.ncell], j3 = (NDIM == 3) ? jc[o + 2 * g.ncell] : (T)0;
   if (jlo) {
     j1 = j1 + jlo[o];
     j2 = j2 + jlo[o + g.ncell];
+    if (NDIM == 3) j3 = j3 + jlo[o + 2 * g.ncell];
   }
-  if (NDIM == 2) {
-    const T* Bz = ebf + 2 * g.ncell;
-    T ex = E1[o] + sdy * (Bz[o] - Bz[o - sy]);
-    T ey = E2[o] - aph1 * (Bz[o] - Bz[o - 1]) - aph2 * (Bz[o + 1] - Bz[o - 2]);
-    if (c.my3) {
-      // curr_mpi_collect on a stretched y: dery (djc jx), derhy (djc jy)
-      E1[o] = ex - ompe * ((T)c.my3[j - 2] * (djc1 * j1));
-      E2[o] = ey - ompe * ((T)c.my4[j - 2] * (djc2 * j2));
-      return;
+  const T e1 = E1[o], e2 = E2[o], e3 = (NDIM == 3) ? E3[o] : (T)0;
+  const T bz = Bz[o], bx = (NDIM == 3) ? Bx[o] : (T)0, by = (NDIM == 3) ? By[o] : (T)0;
+  T bzx, byx = (T)0, bzy, bxy = (T)0, bxz = (T)0, byz = (T)0;  // B one node down along x, y, z
+  const T one = (T)1., two = (T)2.;
+  if (BDS && i == g.ix1) {
+    const T aphx = (T)(1.0 * c.dx_inv * dtl);
+    Bz[o - 1] = bzx = -(two * e2 + (one - aphx) * bz) / (one + aphx);
+    if (NDIM == 3) By[o - 1] = byx = (two * e3 - (one - aphx) * by) / (one + aphx);
+  } else {
+    bzx = Bz[o - 1];
+    if (NDIM == 3) byx = By[o - 1];
+  }
+  if (BDS && j == g.jy1) {
+    const T aphy = (T)(c.by3 * c.dy_inv * dtl);  // loc_yg(1, 3) dy_inv dt
+    const T v = two * e1 - (one - aphy) * bz;
+    Bz[o - sy] = bzy = v / (one + aphy);
+    if (NDIM == 3) {
+      const T w = -two * e3 - (one - aphy) * bx;
+      Bx[o - sy] = bxy = w / (one + aphy);
     }
-    E1[o] = ex - ompe * (djc1 * j1);
-    E2[o] = ey - ompe * (djc2 * j2);
-    return;
+  } else {
+    bzy = Bz[o - sy];
+    if (NDIM == 3) bxy = Bx[o - sy];
   }
-  T* __restrict__ E3 = ebf + 2 * g.ncell;
-  const T* __restrict__ Bx = ebf + 3 * g.ncell;
-  const T* __restrict__ By = ebf + 4 * g.ncell;
-  const T* __restrict__ Bz = ebf + 5 * g.ncell;
-  T j3 = jc[o + 2 * g.ncell];
-  if (jlo) j3 = j3 + jlo[o + 2 * g.ncell];
-  T ex = E1[o] + sdy * (Bz[o] - Bz[o - sy]);
-  T ey = E2[o] - aph1 * (Bz[o] - Bz[o - 1]) - aph2 * (Bz[o + 1] - Bz[o - 2]);
-  ex = ex - sdz * (By[o] - By[o - sz]);
-  ey = ey + sdz * (Bx[o] - Bx[o - sz]);
-  T ez = E3[o] + aph1 * (By[o] - By[o - 1]) - sdy * (Bx[o] - Bx[o - sy]) + aph2 * (By[o + 1] - By[o - 2]);
+  if (NDIM == 3) {
+    if (BDS && k == g.kz1) {
+      const T aphz = (T)(c.bz3 * c.dz_inv * dtl);  // loc_zg(1, 3) dz_inv dt
+      const T v = two * e2 - (one - aphz) * bx;
+      Bx[o - sz] = bxz = v / (one + aphz);
+      const T w = -two * e1 - (one - aphz) * by;
+      By[o - sz] = byz = w / (one + aphz);
+    } else {
+      bxz = Bx[o - sz];
+      byz = By[o - sz];
+    }
+  }
+  T ex = e1 + sdy * (bz - bzy);
+  T ey = e2 - aph1 * (bz - bzx);
+  if (SE2) ey = ey - aph2 * (Bz[o + 1] - Bz[o - 2]);
+  T ez = (T)0;
+  if (NDIM == 3) {
+    ex = ex - sdz * (by - byz);
+    ey = ey + sdz * (bx - bxz);
+    ez = e3 + aph1 * (by - byx) - sdy * (bx - bxy);
+    if (SE2) ez = ez + aph2 * (By[o + 1] - By[o - 2]);
+  }
   if (c.my3) {
-    // curr_mpi_collect on stretched y and z: dery derz, derhy derz, dery derhz
+    // curr_mpi_collect on stretched axes: 2D dery, derhy; 3D dery derz,
+    // derhy derz, dery derhz
     const T dery = (T)c.my3[j - 2], derhy = (T)c.my4[j - 2];
-    const T derz = (T)c.mz3[kn - 2], derhz = (T)c.mz4[kn - 2];
-    E1[o] = ex - ompe * ((dery * derz) * (djc1 * j1));
-    E2[o] = ey - ompe * ((derhy * derz) * (djc2 * j2));
-    E3[o] = ez - ompe * ((dery * derhz) * (djc3 * j3));
+    if (NDIM == 2) {
+      E1[o] = ex - ompe * (dery * (djc1 * j1));
+      E2[o] = ey - ompe * (derhy * (djc2 * j2));
+    } else {
+      const T derz = (T)c.mz3[k - 2], derhz = (T)c.mz4[k - 2];
+      E1[o] = ex - ompe * ((dery * derz) * (djc1 * j1));
+      E2[o] = ey - ompe * ((derhy * derz) * (djc2 * j2));
+      E3[o] = ez - ompe * ((dery * derhz) * (djc3 * j3));
+    }
     return;
   }
   E1[o] = ex - ompe * (djc1 * j1);
   E2[o] = ey - ompe * (djc2 * j2);
-  E3[o] = ez - ompe * (djc3 * j3);
+  if (NDIM == 3) E3[o] = ez - ompe * (djc3 * j3);
+}
+
+// The two sweeps: one thread per node, blocks of 128 x 2 nodes over (i, j)
+// and one z plane per grid layer, so the node indices come without 64-bit
+// divisions.  Measured on the 1024x256x256 grid: the FP32 phase 2.42 -> 2.06
+// ms; marching each thread over several z planes (carrying the z-neighbour
+// loads) was slower.
+constexpr int YEE_BX = 128, YEE_BY = 2;
+
+template <typename T, int NDIM, bool BDS, bool SE2>
+__device__ __forceinline__ void rote_at(T* ebf, const Geo& g, const YeeC& c, double dtf, double dtl, int i, int j, int k) {
+  const double aphxd = dtf * c.dx_inv, aphyd = dtf * c.dy_inv, aphzd = dtf * c.dz_inv;
+  // loc_yg(jj, 4) * aphy, loc_zg(kk, 4) * aphz (1 on a uniform axis)
+  rote_node<T, NDIM, BDS, SE2>(ebf, g, c, goff(g, i, j, k), i, j, k, (T)(aphxd * c.se1), (T)(aphxd * c.se2),
+                               (T)((c.my4 ? c.my4[j - 2] : 1.0) * aphyd),
+                               (T)((c.mz4 && NDIM == 3 ? c.mz4[k - 2] : 1.0) * aphzd), dtl);
+}
+template <typename T, int NDIM, bool BDS, bool SE2>
+__device__ __forceinline__ void rotb_at(T* ebf, const T* jc, const T* jlo, const Geo& g, const YeeC& c, double dtf,
+                                        int i, int j, int k) {
+  const double aphxd = dtf * c.dx_inv, aphyd = dtf * c.dy_inv, aphzd = dtf * c.dz_inv;
+  // loc_yg(jj, 3) * aphy, aphz * loc_zg(kk, 3) (1 on a uniform axis)
+  rotb_node<T, NDIM, BDS, SE2>(ebf, jc, jlo, g, c, goff(g, i, j, k), i, j, k, (T)(aphxd * c.se1), (T)(aphxd * c.se2),
+                               (T)((c.my3 ? c.my3[j - 2] : 1.0) * aphyd),
+                               (T)(aphzd * (c.mz3 && NDIM == 3 ? c.mz3[k - 2] : 1.0)), dtf);
+}
+template <typename T, int NDIM, bool BDS, bool SE2>
+__global__ void __launch_bounds__(YEE_BX* YEE_BY) k_rote(T* ebf, Geo g, YeeC c, double dtf, double dtl) {
+  const int i = g.ix1 + blockIdx.x * YEE_BX + threadIdx.x;
+  const int j = g.jy1 + blockIdx.y * YEE_BY + threadIdx.y;
+  if (i > g.ix2 || j > g.jy2) return;
+  rote_at<T, NDIM, BDS, SE2>(ebf, g, c, dtf, dtl, i, j, (NDIM == 3) ? g.kz1 + (int)blockIdx.z : 1);
+}
+template <typename T, int NDIM, bool BDS, bool SE2>
+__global__ void __launch_bounds__(YEE_BX* YEE_BY) k_rotb_j(T* ebf, const T* jc, const T* jlo, Geo g, YeeC c, double dtf) {
+  const int i = g.ix1 + blockIdx.x * YEE_BX + threadIdx.x;
+  const int j = g.jy1 + blockIdx.y * YEE_BY + threadIdx.y;
+  if (i > g.ix2 || j > g.jy2) return;
+  rotb_at<T, NDIM, BDS, SE2>(ebf, jc, jlo, g, c, dtf, i, j, (NDIM == 3) ? g.kz1 + (int)blockIdx.z : 1);
 }
 
 // ---- comoving frame: field_xadvect (src/fields/grid_fields.f90:210-324) ----
@@ -522,18 +529,38 @@ void yee_t(T* ebf, const T* jc, const T* jlo, const Geo& g, const YeeC& c, cudaS
     if (hk && !hk->rc) hk->rc = hk->fn(hk->ctx, point);
     return hk && hk->rc;
   };
+  // the boundary ghosts ride in the sweeps unless something runs between the
+  // two (a halo exchange, an advection substep) or the wide x difference
+  // reads further out: three launches instead of six (the boundary sweeps
+  // took 4 to 5 us each on every grid)
+  if (!hk && !adv && c.se2 == 0.0) {
+    auto sweeps = [&](auto nd) {
+      constexpr int N = decltype(nd)::value;
+      k_rote<T, N, true, false><<<grd, blk, 0, st>>>(ebf, g, c, dth, 0.0);
+      k_rotb_j<T, N, true, false><<<grd, blk, 0, st>>>(ebf, jc, jlo, g, c, dt);
+      k_rote<T, N, true, false><<<grd, blk, 0, st>>>(ebf, g, c, dth, dt);
+    };
+    if (g.ndim == 3) sweeps(std::integral_constant<int, 3>());
+    else sweeps(std::integral_constant<int, 2>());
+    return;
+  }
+  auto rote = [&]() {
+    if (g.ndim == 3) k_rote<T, 3, false, true><<<grd, blk, 0, st>>>(ebf, g, c, dth, 0.0);
+    else k_rote<T, 2, false, true><<<grd, blk, 0, st>>>(ebf, g, c, dth, 0.0);
+  };
   k_ef_bds<T><<<gf, 256, 0, st>>>(ebf, g, c, 0.0);
   if (halo(AGPU_HALO_E)) return;
   if (adv) xadvect_t<T>(ebf, g, nb1, nb2, 0, *xa, st, sms);
-  if (g.ndim == 3) k_rote_n<T, 3><<<grd, blk, 0, st>>>(ebf, g, c, dth); else k_rote_n<T, 2><<<grd, blk, 0, st>>>(ebf, g, c, dth);
+  rote();
   k_bf_bds<T><<<gf, 256, 0, st>>>(ebf, g, c, dt);
   if (halo(AGPU_HALO_B)) return;
   if (adv) xadvect_t<T>(ebf, g, ne1, ne2, 0, *xa, st, sms);
-  if (g.ndim == 3) k_rotb_j_n<T, 3><<<grd, blk, 0, st>>>(ebf, jc, jlo, g, c, dt); else k_rotb_j_n<T, 2><<<grd, blk, 0, st>>>(ebf, jc, jlo, g, c, dt);
+  if (g.ndim == 3) k_rotb_j<T, 3, false, true><<<grd, blk, 0, st>>>(ebf, jc, jlo, g, c, dt);
+  else k_rotb_j<T, 2, false, true><<<grd, blk, 0, st>>>(ebf, jc, jlo, g, c, dt);
   if (adv) xadvect_t<T>(ebf, g, ne1, ne2, 2, *xa, st, sms);
   k_ef_bds<T><<<gf, 256, 0, st>>>(ebf, g, c, dt);
   if (halo(AGPU_HALO_E)) return;
-  if (g.ndim == 3) k_rote_n<T, 3><<<grd, blk, 0, st>>>(ebf, g, c, dth); else k_rote_n<T, 2><<<grd, blk, 0, st>>>(ebf, g, c, dth);
+  rote();
   if (adv) xadvect_t<T>(ebf, g, nb1, nb2, 2, *xa, st, sms);
 }
 
