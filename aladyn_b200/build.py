@@ -45,7 +45,7 @@ UNITS = [
 ]
 HEADERS = ["agpu_common.cuh", "agpu_kernels.h", "agpu_util.h", "agpu_yee.cuh", "agpu_ionz.h", "agpu_bin.cuh",
            "agpu_tile.h", "agpu_select.cuh", "agpu_beam.h", "agpu_multi.h", "agpu_yee_fused.cuh", "agpu_env.h",
-           "agpu_fp64_dep.cuh", "agpu_tile64.cuh"]
+           "agpu_fp64_dep.cuh", "agpu_tile64.cuh", "agpu_tile32.cuh"]
 
 
 def _mtime(p: str) -> float:

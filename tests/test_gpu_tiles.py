@@ -10,7 +10,7 @@ either sign in another order, each rounded to 2^-53 of at most the largest
 import numpy as np
 import pytest
 
-from aladyn_b200.abi import AGPU_FP64
+from aladyn_b200.abi import AGPU_FP32_SPLIT, AGPU_FP64
 from aladyn_b200.sim import PicDevice, pack_slot
 from oracle.oracle import Oracle
 from tests.helpers import laser_fields, small_case
@@ -22,6 +22,11 @@ CASES = [(2, 31, 7, 1, 700, "spread"), (2, 64, 9, 1, 3000, "piled"), (2, 97, 23,
          (3, 31, 5, 4, 900, "spread"), (3, 33, 6, 7, 4000, "piled"), (3, 70, 13, 9, 30000, "spread")]
 
 
+# every node's octants filled alike: the regular tiles of the split form's
+# one-node-per-thread path, and the last, partial ones
+LATTICE = (3, 66, 9, 9, 8 * 66 * 9 * 9, "lattice")
+
+
 def records(p, n, how, pmax, seed=3):
     r = np.random.default_rng(seed)
     nd = p.ndim
@@ -29,6 +34,10 @@ def records(p, n, how, pmax, seed=3):
     rec = np.zeros((n, 2 * nd + 1), order="F")
     for a in range(nd):
         u = r.random(n)
+        if how == "lattice":
+            cells = [p.nx, p.ny, p.nz]
+            q = np.arange(n) // int(np.prod([2 * c for c in cells[:a]], dtype=np.int64)) % (2 * cells[a])
+            u = (q + 0.4 + 0.2 * u) / (2 * cells[a])
         if how == "piled":  # half of the records in one cell, the rest in a few
             u = np.where(r.random(n) < 0.5, 0.4 + 0.002 * u, 0.35 + 0.15 * u)
         rec[:, a] = lo[a] + (hi[a] - lo[a]) * (1e-9 + (1 - 2e-9) * u)
@@ -56,6 +65,28 @@ def test_fp64_tile_step(ndim, nx, ny, nz, n, how, pmax):
     assert np.array_equal(a.view(np.uint64), b.view(np.uint64))
     ja, jb = dev.get_currents(), ora.get_currents()
     assert np.abs(ja - jb).max() <= 1e-12 * np.abs(jb).max()
+
+
+@pytest.mark.parametrize("pmax", [0.05, 5.0])
+@pytest.mark.parametrize("ndim,nx,ny,nz,n,how", CASES + [LATTICE])
+def test_split_tile_step(ndim, nx, ny, nz, n, how, pmax):
+    """The split form.  A record's offsets are rounded to
+    2^-25 cells and each current term to a few times 2^-24 of q w, so against
+    displacements of 0.02 cells and more (pmax = 0.05) the currents are off by
+    less than 1e-4 of their norm; positions by 2^-24 of a cell, momenta by a
+    few 2^-24 of the largest one."""
+    got = []
+    for cls, prec in ((PicDevice, AGPU_FP32_SPLIT), (Oracle, AGPU_FP64)):
+        p = small_case(ndim, nx=nx, ny=ny, nz=nz, cap=n + 16, precision=prec)
+        d = step(cls, p, records(p, n, how, pmax), laser_fields(p))
+        got.append((d.get_species(0), d.get_currents()))
+    (a, ja), (b, jb) = got
+    assert a.shape == b.shape
+    cell = [p.dx, p.dy, p.dz]
+    for c in range(ndim):
+        assert np.abs(a[:, c] - b[:, c]).max() <= 4e-7 * cell[c]
+        assert np.abs(a[:, ndim + c] - b[:, ndim + c]).max() <= 4e-6 * np.abs(b[:, ndim:2 * ndim]).max()
+    assert np.linalg.norm(ja - jb) <= 1e-4 * np.linalg.norm(jb)
 
 
 def env_step(cls, p, ep, rec, ebf, env0, nsteps):
