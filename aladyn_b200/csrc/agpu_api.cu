@@ -573,6 +573,11 @@ int reorder_records(agpu_handle* h, int ic) {
   return 0;
 }
 
+HistReset hist_args(agpu_handle* h, int ic) {
+  return HistReset{h->hist[ic],     h->tstart[ic], h->tg.nkeys, (int)h->np[ic], h->defer ? &h->d_cnt->pushed : nullptr,
+                   h->tile_work_n};
+}
+
 // Arguments of the FP64 tile kernels for species ic.
 void tile_args64(const agpu_handle* h, int ic, int initial_time, TileArgs64& a) {
   const agpu_params& p = h->p;
@@ -621,10 +626,11 @@ void tile_args64(const agpu_handle* h, int ic, int initial_time, TileArgs64& a) 
   a.err = &h->d_cnt->err;
 }
 
-// Tiled gather + push + deposit of species ic, then the next binning from
+// Tiled gather + push + deposit of species ic (hist_done: the histogram is
+// reset already), then the next binning from
 // the keys the kernel wrote.  Removed particles stay stored (key nkeys)
 // until the next compaction.
-int tiled_push(agpu_handle* h, int ic, int initial_time) {
+int tiled_push(agpu_handle* h, int ic, int initial_time, bool hist_done) {
   const agpu_params& p = h->p;
   if (!h->binned[ic]) {
     ph_begin(h, PH_SORT);
@@ -633,7 +639,7 @@ int tiled_push(agpu_handle* h, int ic, int initial_time) {
     if (rc) return rc;
   }
   const long long alive0 = h->nalive[ic];
-  hist_reset(h->hist[ic], h->tstart[ic], h->tg, h->np[ic], h->defer ? &h->d_cnt->pushed : nullptr, h->tile_work_n, h->st);
+  if (!hist_done) hist_reset(hist_args(h, ic), h->st);
   ph_begin(h, PH_PUSH);
   if (h->fp32) {
     TileArgs32 a;
@@ -670,7 +676,7 @@ int tiled_push(agpu_handle* h, int ic, int initial_time) {
   CK(cudaGetLastError());
   ph_end(h, PH_PUSH);
   h->timers.launches_push_deposit += 1;
-  h->timers.launches_total += 2;  // histogram reset + tile kernel
+  h->timers.launches_total += hist_done ? 1 : 2;  // histogram reset + tile kernel
   if (!h->defer) h->timers.pushes += alive0;
   ph_begin(h, PH_SORT);
   const int nl = bin_finish(h->key[ic], h->np[ic], h->tg, h->hist[ic], h->tstart[ic], h->cursor, h->perm[ic], h->scan_tmp,
@@ -1781,10 +1787,16 @@ static int step_impl(agpu_handle* h, int32_t iter, double t, int32_t initial_tim
   } else {
     CK(cudaMemsetAsync(h->d_cnt, 0, sizeof(Counters), h->st));
   }
-  // pfields_prepare -> field_xyzbd
+  // pfields_prepare -> field_xyzbd; with one tiled species, binned by the
+  // step before, jc = 0 and its histogram reset in the same launch
+  const bool pre = p.nsp_run == 1 && p.ionz_lev == 0 && h->np[0] > 0 && h->binned[0] && tiled(h, 0);
   ph_begin(h, PH_YEE);
-  if (h->fp32) field_bd32(Dev32{h->g, h->ebf32, h->jhi, h->jlo}, h->st, h->sms);
-  else field_bd64(Dev64{h->g, h->ebf, h->jc}, h->st, h->sms);
+  const Dev32 d32{h->g, h->ebf32, h->jhi, h->jlo};
+  const Dev64 d64{h->g, h->ebf, h->jc};
+  if (pre && h->fp32) step_pre32(d32, hist_args(h, 0), h->st, h->sms);
+  else if (pre) step_pre64(d64, hist_args(h, 0), h->st, h->sms);
+  else if (h->fp32) field_bd32(d32, h->st, h->sms);
+  else field_bd64(d64, h->st, h->sms);
   CK(cudaGetLastError());
   h->timers.launches_total += 1;
   if (int rc_ = halo_call(h, AGPU_HALO_FIELDS, -1)) return rc_;
@@ -1797,7 +1809,8 @@ static int step_impl(agpu_handle* h, int32_t iter, double t, int32_t initial_tim
     if (rc) return rc;
   }
   // jc = 0, then each running species: gather/push/deposit
-  if (h->fp32) {
+  if (pre) {
+  } else if (h->fp32) {
     CK(cudaMemsetAsync(h->jhi, 0, sizeof(float) * h->g.ncell * h->g.nc, h->st));
     CK(cudaMemsetAsync(h->jlo, 0, sizeof(float) * h->g.ncell * h->g.nc, h->st));
   } else {
@@ -1811,7 +1824,7 @@ static int step_impl(agpu_handle* h, int32_t iter, double t, int32_t initial_tim
       continue;
     }
     if (tiled(h, ic)) {
-      if (int rc_ = tiled_push(h, ic, initial_time)) return rc_;
+      if (int rc_ = tiled_push(h, ic, initial_time, pre)) return rc_;
       if (sort_step(h, iter)) {
         if (int rc_ = settle_counts(h, out)) return rc_;
         if (int rc_ = reorder_records(h, ic)) return rc_;
@@ -1950,7 +1963,7 @@ static int step_impl(agpu_handle* h, int32_t iter, double t, int32_t initial_tim
   ph_end(h, PH_YEE);
   h->timers.launches_yee += 1;
   // current fold + the Yee kernels
-  h->timers.launches_total += 1 + (fused ? 1 : yee_launches(c, h->dd || h->xadv.tmp)) + xadv_launches(h);
+  h->timers.launches_total += (p.ndim == 3 ? 3 : 1) + (fused ? 1 : yee_launches(c, h->dd || h->xadv.tmp)) + xadv_launches(h);
   h->timers.yee_cells += (long long)p.nx * p.ny * (p.ndim == 3 ? p.nz : 1);
   // lp_run: moving window, or the comoving frame's coordinate shift.  The
   // counts come over once, after the last kernel of a plain step or before
@@ -2370,7 +2383,9 @@ int agpu_env_run(agpu_handle* h, int32_t iter, double t, agpu_step_out* out) {
     tile_args64(h, ic, 0, ta);
     ta.av = h->env_av;
     ta.den = h->env_den;
-    hist_reset(h->hist[ic], h->tstart[ic], h->tg, h->np[ic], nullptr, nullptr, h->st);
+    HistReset hr = hist_args(h, ic);
+    hr.pushed = nullptr;  // counted by the host
+    hist_reset(hr, h->st);
   }
   // set_env_acc, lpf_env_momenta, set_env_density (jc(:,:,:,1) = 0 first)
   CK(cudaMemsetAsync(h->env_den, 0, sizeof(double) * c3, h->st));
@@ -2422,7 +2437,7 @@ int agpu_env_run(agpu_handle* h, int32_t iter, double t, agpu_step_out* out) {
   CK(cudaGetLastError());
   ph_end(h, PH_YEE);
   h->timers.launches_yee += 1;
-  h->timers.launches_total += 1 + yee_launches(yee_coef(p), h->xadv.tmp != nullptr) + xadv_launches(h);
+  h->timers.launches_total += (p.ndim == 3 ? 3 : 1) + yee_launches(yee_coef(p), h->xadv.tmp != nullptr) + xadv_launches(h);
   h->timers.yee_cells += (long long)p.nx * p.ny * (p.ndim == 3 ? p.nz : 1);
   if ((rc = window_or_comoving(h, iter, t, out, true))) return rc;
   if (int rc_ = read_counters(h)) return rc_;

@@ -61,6 +61,25 @@ __device__ __forceinline__ void hist_add(int* hist, int key) {
   if ((threadIdx.x & 31) == leader) atomicAdd(&hist[key], __popc(peers));
 }
 
+// The next histogram's reset: bins zero, the dead bin seeded with the records
+// already dead (no tile visits them); with `pushed` set, the alive count of
+// this push (tstart[nkeys]) is added to it (the deferred-count mode keeps the
+// push count on the device); the split form's work-list counters cleared.
+struct HistReset {
+  int* hist;
+  const int* tstart;
+  int nkeys, np;
+  unsigned long long* pushed;
+  unsigned int* work_n;
+};
+__device__ __forceinline__ void hist_reset_bin(const HistReset& h, int b) {
+  if (h.work_n && b < 2) h.work_n[b] = 0u;
+  if (b > h.nkeys) return;
+  const int alive = (b == h.nkeys) ? h.tstart[b] : 0;
+  h.hist[b] = (b == h.nkeys) ? h.np - alive : 0;
+  if (b == h.nkeys && h.pushed) *h.pushed += (unsigned long long)alive;
+}
+
 struct Scratch;
 struct Part32View;
 void bin_keys_split(const int* cell, const float* ox, const float* oy, const float* oz, long long np, const Geo& g,

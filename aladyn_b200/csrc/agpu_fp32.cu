@@ -14,9 +14,12 @@
 
 namespace agpu {
 
-void field_bd32(const Dev32& d, cudaStream_t st, int sms) { field_bd_t<float>(d.ebf, d.g, st, sms); }
+void step_pre32(const Dev32& d, const HistReset& h, cudaStream_t st, int sms) {
+  step_pre_t<float>(d.ebf, d.jhi, d.jlo, d.g, h, st, sms);
+}
+void field_bd32(const Dev32& d, cudaStream_t st, int sms) { field_bd_t<float>(d.ebf, d.g, st); }
 void jfold32(const Dev32& d, cudaStream_t st, int sms) {
-  jfold_t<float>(d.jhi, d.jlo, d.g, st, sms);
+  jfold_t<float>(d.jhi, d.jlo, d.g, st);
 }
 void yee32(const Dev32& d, const YeeC& c, cudaStream_t st, int sms) { yee_t<float>(d.ebf, d.jhi, d.jlo, d.g, c, st, sms); }
 void yee32_fused(const float* fin, float* fout, const float* jhi, const float* jlo, const Geo& g, const YeeC& c,
@@ -442,11 +445,18 @@ __global__ void km_pre(const MultiInst* __restrict__ d) {
       m.ta.hist[b] = 0;
     }
   }
-  d_field_bd<float>(m.ebf, g, g.nf, bid_, nb_);
+  const int nbd = bd_nodes(g);
+  for (int c = 0; c < g.nf; ++c)
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nbd; r += gridDim.x * blockDim.x)
+      field_bd_node(m.ebf + g.ncell * c, g, r);
 }
 __global__ void km_fold(const MultiInst* __restrict__ d) {
   const MultiInst& m = d[blockIdx.y];
-  d_jfold<float>(m.ta.jhi, m.ta.jlo, m.ta.g, blockIdx.x, gridDim.x);
+  const Geo g = m.ta.g;
+  float *hi = m.ta.jhi, *lo = m.ta.jlo;
+  const int n = fold_nodes(g);
+  for (int q = 0; q < 2 * g.nc; ++q)
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) jfold_node(hi, lo, g, q, r);
 }
 __global__ void km_ef_bds(const MultiInst* __restrict__ d, int full_dt) {
   const MultiInst& m = d[blockIdx.y];

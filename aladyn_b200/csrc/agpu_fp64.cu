@@ -13,7 +13,10 @@
 
 namespace agpu {
 
-void field_bd64(const Dev64& d, cudaStream_t st, int sms) { field_bd_t<double>(d.ebf, d.g, st, sms); }
+void step_pre64(const Dev64& d, const HistReset& h, cudaStream_t st, int sms) {
+  step_pre_t<double>(d.ebf, d.jc, nullptr, d.g, h, st, sms);
+}
+void field_bd64(const Dev64& d, cudaStream_t st, int sms) { field_bd_t<double>(d.ebf, d.g, st); }
 
 // ============================================================================
 // Cubic shape extension (AGPU_SHAPE_CUBIC; no counterpart in the reference):
@@ -514,7 +517,7 @@ void push_deposit64(const PushArgs64& a, cudaStream_t st, int sms, bool serial) 
   }
 }
 
-void jfold64(const Dev64& d, cudaStream_t st, int sms) { jfold_t<double>(d.jc, (double*)nullptr, d.g, st, sms); }
+void jfold64(const Dev64& d, cudaStream_t st, int sms) { jfold_t<double>(d.jc, (double*)nullptr, d.g, st); }
 
 void yee64(const Dev64& d, const YeeC& c, cudaStream_t st, int sms, const XAdv* xa, YeeHook* hk) {
   yee_t<double>(d.ebf, d.jc, (const double*)nullptr, d.g, c, st, sms, xa, hk);

@@ -116,7 +116,10 @@ struct IonArgs64 {
   unsigned int* err;
 };
 
+struct HistReset;
 void field_bd64(const Dev64& d, cudaStream_t st, int sms);
+// field_bd, jc = 0 and the histogram reset of the one tiled species
+void step_pre64(const Dev64& d, const HistReset& h, cudaStream_t st, int sms);
 void push_deposit64(const PushArgs64& a, cudaStream_t st, int sms, bool serial);
 void jfold64(const Dev64& d, cudaStream_t st, int sms);
 void yee64(const Dev64& d, const YeeC& c, cudaStream_t st, int sms, const XAdv* xa = nullptr, YeeHook* hk = nullptr);
@@ -181,6 +184,7 @@ __global__ void k32_ion_efield(IonArgs32 a);
 __global__ void k32_ionize(IonArgs32 a);
 
 void field_bd32(const Dev32& d, cudaStream_t st, int sms);
+void step_pre32(const Dev32& d, const HistReset& h, cudaStream_t st, int sms);
 void push_deposit32(const PushArgs32& a, cudaStream_t st, int sms);
 void jfold32(const Dev32& d, cudaStream_t st, int sms);
 void yee32(const Dev32& d, const YeeC& c, cudaStream_t st, int sms);

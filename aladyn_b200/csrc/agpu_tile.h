@@ -71,7 +71,6 @@ void tile_push32_cubic(const TileArgs32& a, cudaStream_t st);
 void tile_push64(const TileArgs64& a, cudaStream_t st);
 void env_acc_tile(const EnvTileArgs& a, cudaStream_t st);
 void env_pos_tile(const EnvTileArgs& a, cudaStream_t st);
-void hist_reset(int* hist, const int* tstart, const TileGeo& t, long long np, unsigned long long* pushed,
-                unsigned int* work_n, cudaStream_t st);
+void hist_reset(const HistReset& h, cudaStream_t st);
 
 }  // namespace agpu

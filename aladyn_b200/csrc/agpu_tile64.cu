@@ -236,22 +236,8 @@ void tile_push64(const TileArgs64& a, cudaStream_t st) {
   else tile_push64_t<2>(a, st);
 }
 
-// Next histogram zeroed, the dead bin seeded with the records already dead
-// (no tile visits them); with `pushed` set, the alive count of this push
-// (tstart[nkeys]) is added to it (the deferred-count mode keeps the push
-// count on the device); the split form's work-list counters cleared.
-__global__ void k_hist_reset(int* hist, const int* tstart, int nkeys, int np, unsigned long long* pushed,
-                             unsigned int* work_n) {
-  if (work_n && blockIdx.x == 0 && threadIdx.x < 2) work_n[threadIdx.x] = 0u;
-  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b <= nkeys; b += gridDim.x * blockDim.x) {
-    hist[b] = (b == nkeys) ? (np - tstart[nkeys]) : 0;
-    if (b == nkeys && pushed) *pushed += (unsigned long long)tstart[nkeys];
-  }
-}
-void hist_reset(int* hist, const int* tstart, const TileGeo& t, long long np, unsigned long long* pushed,
-                unsigned int* work_n, cudaStream_t st) {
-  k_hist_reset<<<(t.nkeys + 256) / 256, 256, 0, st>>>(hist, tstart, t.nkeys, (int)np, pushed, work_n);
-}
+__global__ void k_hist_reset(HistReset h) { hist_reset_bin(h, blockIdx.x * blockDim.x + threadIdx.x); }
+void hist_reset(const HistReset& h, cudaStream_t st) { k_hist_reset<<<(h.nkeys + 256) / 256, 256, 0, st>>>(h); }
 
 TileGeo make_tiles(const Geo& g, int nx, int ny, int nz, bool fp32) {
   TileGeo t;

@@ -7,6 +7,7 @@
 #include <type_traits>
 
 #include "agpu_common.cuh"
+#include "agpu_bin.cuh"
 #include "agpu_kernels.h"
 
 namespace agpu {
@@ -47,14 +48,12 @@ AGPU_HD int bd_nodes(const Geo& g) {
   const int nx = g.ix2 - g.ix1 + 1, ny = g.jy2 - g.jy1 + 1, nz = g.kz2 - g.kz1 + 1;
   return 2 * (ny * nz + (nx + 2) * nz + (g.ndim == 3 ? (nx + 2) * (ny + 2) : 0));
 }
+// ghost node r of component f
 template <typename T>
-__device__ __forceinline__ void d_field_bd(T* ebf, const Geo& g, int nc, long long bid_, long long nb_) {
+__device__ __forceinline__ void field_bd_node(T* f, const Geo& g, int r) {
   const int nxe = g.ix2 - g.ix1 + 3, nye = g.jy2 - g.jy1 + 3, ny = nye - 2, nz = g.kz2 - g.kz1 + 1;
-  const int n = bd_nodes(g), fx = 2 * ny * nz, fy = 2 * nxe * nz;
-  GRID_STRIDE(t, (long long)n * nc) {
-    const int ik = (int)(t / n);
-    int r = (int)(t - (long long)ik * n);
-    T* f = ebf + g.ncell * ik;
+  const int fx = 2 * ny * nz, fy = 2 * nxe * nz;
+  {
     int i, j, k;
     T v;
     if (r < fx) {
@@ -84,13 +83,46 @@ __device__ __forceinline__ void d_field_bd(T* ebf, const Geo& g, int nc, long lo
     f[goff(g, i, j, k)] = v;
   }
 }
+// one thread per node, one grid row per component
 template <typename T>
-__global__ void k_field_bd(T* ebf, Geo g, int nc) {
-  d_field_bd<T>(ebf, g, nc, blockIdx.x, gridDim.x);
+__global__ void k_field_bd(T* ebf, Geo g) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r < bd_nodes(g)) field_bd_node(ebf + g.ncell * blockIdx.y, g, r);
 }
 template <typename T>
-void field_bd_t(T* ebf, const Geo& g, cudaStream_t st, int sms) {
-  k_field_bd<T><<<grid_for((long long)bd_nodes(g) * g.nf, 256, sms), 256, 0, st>>>(ebf, g, g.nf);
+void field_bd_t(T* ebf, const Geo& g, cudaStream_t st) {
+  k_field_bd<T><<<dim3((bd_nodes(g) + 255) / 256, g.nf), 256, 0, st>>>(ebf, g);
+}
+
+// What a step clears before its push, in one launch with the field
+// extrapolation: the currents (both parts) and the next histogram
+// (hist_reset).  On small grids each of the four launches it replaces cost
+// about 3 us.  Block ranges: ghost nodes, histogram, currents (nzero blocks).
+template <typename T>
+__global__ void k_step_pre(T* ebf, Geo g, T* j0, T* j1, HistReset h, int bbd, int bhist, int nzero) {
+  int b = blockIdx.x;
+  if (b < bbd * g.nf) {
+    const int c = b / bbd, r = (b - c * bbd) * blockDim.x + threadIdx.x;
+    if (r < bd_nodes(g)) field_bd_node(ebf + g.ncell * c, g, r);
+    return;
+  }
+  b -= bbd * g.nf;
+  if (b < bhist) {
+    hist_reset_bin(h, b * blockDim.x + threadIdx.x);
+    return;
+  }
+  b -= bhist;
+  const long long n = g.ncell * g.nc;
+  for (long long q = b * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)nzero * blockDim.x) {
+    j0[q] = (T)0;
+    if (j1) j1[q] = (T)0;
+  }
+}
+template <typename T>
+void step_pre_t(T* ebf, T* j0, T* j1, const Geo& g, const HistReset& h, cudaStream_t st, int sms) {
+  const int bbd = (bd_nodes(g) + 255) / 256, bhist = (h.nkeys + 256) / 256;
+  const int nzero = grid_for(g.ncell * g.nc, 256, sms, 16);
+  k_step_pre<T><<<bbd * g.nf + bhist + nzero, 256, 0, st>>>(ebf, g, j0, j1, h, bbd, bhist, nzero);
 }
 
 // ---- A13: jc_xyzbd (src/parallel/mpi_curr_interface.f90:551-643) ----------
@@ -104,14 +136,13 @@ AGPU_HD int fold_nodes(const Geo& g) {
   const int nx = g.ix2 - g.ix1 + 1, ny = g.jy2 - g.jy1 + 1, nz = g.kz2 - g.kz1 + 1;
   return 2 * (ny * nz + (nx - 2) * nz + (g.ndim == 3 ? (nx - 2) * (ny - 2) : 0));
 }
+// boundary node r of component q (j0's components, then j1's)
 template <typename T>
-__device__ __forceinline__ void d_jfold(T* j0, T* j1, const Geo& g, long long bid_, long long nb_) {
+__device__ __forceinline__ void jfold_node(T* j0, T* j1, const Geo& g, int q, int r) {
   const int nx = g.ix2 - g.ix1 + 1, ny = g.jy2 - g.jy1 + 1, nz = g.kz2 - g.kz1 + 1;
-  const int n = fold_nodes(g), fx = 2 * ny * nz, fy = 2 * (nx - 2) * nz;
+  const int fx = 2 * ny * nz, fy = 2 * (nx - 2) * nz;
   const long long sy = g.n1p, sz = (long long)g.n1p * g.n2p;
-  GRID_STRIDE(t, (long long)n * g.nc * (j1 ? 2 : 1)) {
-    const int q = (int)(t / n);
-    int r = (int)(t - (long long)q * n);
+  {
     int i, j, k;
     if (r < fx) {
       const int hi = r >= fx / 2;
@@ -159,12 +190,50 @@ __device__ __forceinline__ void d_jfold(T* j0, T* j1, const Geo& g, long long bi
 }
 template <typename T>
 __global__ void k_jfold(T* j0, T* j1, Geo g) {
-  d_jfold<T>(j0, j1, g, blockIdx.x, gridDim.x);
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r < fold_nodes(g)) jfold_node(j0, j1, g, blockIdx.y, r);
 }
-// j1: the compensation part of a two-float current, or null
+// One axis of the fold: both of its faces, all interior nodes of the other
+// two axes.
+template <typename T, int AX>
+__global__ void k_jfold_axis(T* j0, T* j1, Geo g) {
+  const int nx = g.ix2 - g.ix1 + 1, ny = g.jy2 - g.jy1 + 1, nz = g.kz2 - g.kz1 + 1;
+  const int m = (AX == 0) ? ny : nx, n = m * ((AX == 2) ? ny : nz);
+  int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= 2 * n) return;
+  const int hi = r >= n;
+  r -= hi * n;
+  const int u = r % m, v = r / m;
+  const int i = (AX == 0) ? (hi ? g.ix2 : g.ix1) : g.ix1 + u;
+  const int j = (AX == 1) ? (hi ? g.jy2 : g.jy1) : g.jy1 + (AX == 0 ? u : v);
+  const int k = (AX == 2) ? (hi ? g.kz2 : g.kz1) : g.kz1 + v;
+  const int q = blockIdx.y;
+  T* c = (q < g.nc ? j0 + g.ncell * q : j1 + g.ncell * (q - g.nc)) + goff(g, i, j, k);
+  const long long s = (AX == 0) ? 1 : (AX == 1) ? g.n1p : (long long)g.n1p * g.n2p, d = hi ? s : -s;
+  const T a = c[0], b = c[d];
+  c[d] = (T)0;
+  if (hi || AX == 1) {
+    c[0] = a + b + c[2 * d];
+    c[2 * d] = (T)0;
+  } else {
+    c[0] = a + b;
+  }
+}
+// j1: the compensation part of a two-float current, or null.  2D in one sweep
+// (4 us against 8: launches are what counts); in 3D one launch per axis: the
+// one sweep took 60 us on 384x96x96 cells, the axes' launches 5 each.
 template <typename T>
-void jfold_t(T* j0, T* j1, const Geo& g, cudaStream_t st, int sms) {
-  k_jfold<T><<<grid_for((long long)fold_nodes(g) * g.nc * (j1 ? 2 : 1), 256, sms), 256, 0, st>>>(j0, j1, g);
+void jfold_t(T* j0, T* j1, const Geo& g, cudaStream_t st) {
+  const int nq = g.nc * (j1 ? 2 : 1);
+  if (g.ndim == 2) {
+    k_jfold<T><<<dim3((fold_nodes(g) + 255) / 256, nq), 256, 0, st>>>(j0, j1, g);
+    return;
+  }
+  const int nx = g.ix2 - g.ix1 + 1, ny = g.jy2 - g.jy1 + 1, nz = g.kz2 - g.kz1 + 1;
+  auto blocks = [&](int n) { return dim3((2 * n + 255) / 256, nq); };
+  k_jfold_axis<T, 0><<<blocks(ny * nz), 256, 0, st>>>(j0, j1, g);
+  k_jfold_axis<T, 1><<<blocks(nx * nz), 256, 0, st>>>(j0, j1, g);
+  k_jfold_axis<T, 2><<<blocks(nx * ny), 256, 0, st>>>(j0, j1, g);
 }
 
 // ---- A14: Yee (advance_lpf_fields, curr_and_fields_util.f90:176-260) ------
@@ -274,7 +343,8 @@ __device__ __forceinline__ void rote_node(T* ebf, const Geo& g, const YeeC& c, l
   T* Bx = ebf + 3 * g.ncell;
   T* By = ebf + 4 * g.ncell;
   T* Bz = ebf + (NDIM == 3 ? 5 : 2) * g.ncell;
-  const T e1 = E1[o], e2 = E2[o], e3 = (NDIM == 3) ? E3[o] : (T)0;
+  // the sweep writes no E that another node reads: read-only loads
+  const T e1 = __ldg(E1 + o), e2 = __ldg(E2 + o), e3 = (NDIM == 3) ? __ldg(E3 + o) : (T)0;
   const T bz = Bz[o], bx = (NDIM == 3) ? Bx[o] : (T)0, by = (NDIM == 3) ? By[o] : (T)0;
   T e2x, e3x = (T)0, e1y, e3y = (T)0, e1z = (T)0, e2z = (T)0;  // E one node up along x, y, z
   const T one = (T)1., two = (T)2.;
@@ -283,16 +353,16 @@ __device__ __forceinline__ void rote_node(T* ebf, const Geo& g, const YeeC& c, l
     E2[o + 1] = e2x = (two * bz - (one - aphx) * e2) / (one + aphx);
     if (NDIM == 3) E3[o + 1] = e3x = -(two * by + (one - aphx) * e3) / (one + aphx);
   } else {
-    e2x = E2[o + 1];
-    if (NDIM == 3) e3x = E3[o + 1];
+    e2x = __ldg(E2 + o + 1);
+    if (NDIM == 3) e3x = __ldg(E3 + o + 1);
   }
   if (BDS && j == g.jy2) {
     const T aphy = (T)(c.ty4 * c.dy_inv * dtl);  // loc_yg(ny, 4) dy_inv dt
     E1[o + sy] = e1y = -(two * bz + (one - aphy) * e1) / (one + aphy);
     if (NDIM == 3) E3[o + sy] = e3y = (two * bx - (one - aphy) * e3) / (one + aphy);
   } else {
-    e1y = E1[o + sy];
-    if (NDIM == 3) e3y = E3[o + sy];
+    e1y = __ldg(E1 + o + sy);
+    if (NDIM == 3) e3y = __ldg(E3 + o + sy);
   }
   if (NDIM == 3) {
     if (BDS && k == g.kz2) {
@@ -300,8 +370,8 @@ __device__ __forceinline__ void rote_node(T* ebf, const Geo& g, const YeeC& c, l
       E1[o + sz] = e1z = (two * by - (one - aphz) * e1) / (one + aphz);
       E2[o + sz] = e2z = -(two * bx + (one - aphz) * e2) / (one + aphz);
     } else {
-      e1z = E1[o + sz];
-      e2z = E2[o + sz];
+      e1z = __ldg(E1 + o + sz);
+      e2z = __ldg(E2 + o + sz);
     }
   }
   const T nz = bz - aph1 * (e2x - e2) + sdhy * (e1y - e1);
@@ -329,14 +399,15 @@ __device__ __forceinline__ void rotb_node(T* ebf, const T* jc, const T* jlo, con
   T* By = ebf + 4 * g.ncell;
   T* Bz = ebf + (NDIM == 3 ? 5 : 2) * g.ncell;
   const T ompe = (T)c.ompe, djc1 = (T)c.djc1, djc2 = (T)c.djc2, djc3 = (T)c.djc3;
-  T j1 = jc[o], j2 = jc[o + g.ncell], j3 = (NDIM == 3) ? jc[o + 2 * g.ncell] : (T)0;
+  T j1 = __ldg(jc + o), j2 = __ldg(jc + o + g.ncell), j3 = (NDIM == 3) ? __ldg(jc + o + 2 * g.ncell) : (T)0;
   if (jlo) {
-    j1 = j1 + jlo[o];
-    j2 = j2 + jlo[o + g.ncell];
-    if (NDIM == 3) j3 = j3 + jlo[o + 2 * g.ncell];
+    j1 = j1 + __ldg(jlo + o);
+    j2 = j2 + __ldg(jlo + o + g.ncell);
+    if (NDIM == 3) j3 = j3 + __ldg(jlo + o + 2 * g.ncell);
   }
   const T e1 = E1[o], e2 = E2[o], e3 = (NDIM == 3) ? E3[o] : (T)0;
-  const T bz = Bz[o], bx = (NDIM == 3) ? Bx[o] : (T)0, by = (NDIM == 3) ? By[o] : (T)0;
+  // the sweep writes no B that another node reads
+  const T bz = __ldg(Bz + o), bx = (NDIM == 3) ? __ldg(Bx + o) : (T)0, by = (NDIM == 3) ? __ldg(By + o) : (T)0;
   T bzx, byx = (T)0, bzy, bxy = (T)0, bxz = (T)0, byz = (T)0;  // B one node down along x, y, z
   const T one = (T)1., two = (T)2.;
   if (BDS && i == g.ix1) {
@@ -344,8 +415,8 @@ __device__ __forceinline__ void rotb_node(T* ebf, const T* jc, const T* jlo, con
     Bz[o - 1] = bzx = -(two * e2 + (one - aphx) * bz) / (one + aphx);
     if (NDIM == 3) By[o - 1] = byx = (two * e3 - (one - aphx) * by) / (one + aphx);
   } else {
-    bzx = Bz[o - 1];
-    if (NDIM == 3) byx = By[o - 1];
+    bzx = __ldg(Bz + o - 1);
+    if (NDIM == 3) byx = __ldg(By + o - 1);
   }
   if (BDS && j == g.jy1) {
     const T aphy = (T)(c.by3 * c.dy_inv * dtl);  // loc_yg(1, 3) dy_inv dt
@@ -356,8 +427,8 @@ __device__ __forceinline__ void rotb_node(T* ebf, const T* jc, const T* jlo, con
       Bx[o - sy] = bxy = w / (one + aphy);
     }
   } else {
-    bzy = Bz[o - sy];
-    if (NDIM == 3) bxy = Bx[o - sy];
+    bzy = __ldg(Bz + o - sy);
+    if (NDIM == 3) bxy = __ldg(Bx + o - sy);
   }
   if (NDIM == 3) {
     if (BDS && k == g.kz1) {
@@ -367,8 +438,8 @@ __device__ __forceinline__ void rotb_node(T* ebf, const T* jc, const T* jlo, con
       const T w = -two * e1 - (one - aphz) * by;
       By[o - sz] = byz = w / (one + aphz);
     } else {
-      bxz = Bx[o - sz];
-      byz = By[o - sz];
+      bxz = __ldg(Bx + o - sz);
+      byz = __ldg(By + o - sz);
     }
   }
   T ex = e1 + sdy * (bz - bzy);

@@ -36,7 +36,7 @@ def test_boundaries_bitexact(ndim, nx, ny, nz, der_ord):
 
 @pytest.mark.parametrize("nx,ny", [(64, 9), (1000, 250), (2100, 260)])
 def test_key_scan_sizes(nx, ny):
-    """288, 64512 and 139392 + 1 keys: every particle is in the tiles once,
+    """193, 32769 and 69697 keys: every particle is in the tiles once,
     so the step keeps the count and the particles stay bit-exact."""
     p = small_case(2, nx=nx, ny=ny, cap=60000, w_sh=0)
     rec, ebf = records(p, 50000, "spread", 0.05), laser_fields(p)
