@@ -1,6 +1,6 @@
 // agpu_tile32.cu — tiled gather + push + deposit of the FP32 split form with
 // the reference's quadratic shapes, on the tile step of agpu_tile32.cuh.
-// Bound: instruction latency at 16 warps per SM (46 % of the issue slots,
+// Bound: instruction latency at 16 warps per SM (43 % of the issue slots,
 // DRAM traffic the algorithmic 76 B a particle).  The earlier kernel, one node
 // per thread throughout, ran its warps with 25 of 32 lanes in a driven plasma
 // (384x96x96 cells, 2.8e7 electrons): a pass of 10 steps 39.6 ms against 34.4

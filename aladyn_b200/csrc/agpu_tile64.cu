@@ -1,6 +1,6 @@
 // agpu_tile64.cu — tiled gather + push + deposit of the plain FP64 form, on
 // the tile step of agpu_tile64.cuh.  Bound: FP64 latency and shared-memory
-// bandwidth at 16 warps per SM (FP64 pipe 41 % busy, LSU 60 %), no longer L2
+// bandwidth at 16 warps per SM (FP64 pipe 41 % busy, LSU 56 %), no longer L2
 // atomics: the earlier deposit, one particle per lane with 81 global FP64
 // atomics each (4.2e11 atomics/s), took 4.5 ms a step for 1.88e7 electrons
 // in a laser-driven plasma (256x96x96 cells) against 2.4 ms now; 2D
