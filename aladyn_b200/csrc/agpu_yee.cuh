@@ -194,7 +194,10 @@ __global__ void k_jfold(T* j0, T* j1, Geo g) {
   if (r < fold_nodes(g)) jfold_node(j0, j1, g, blockIdx.y, r);
 }
 // One axis of the fold: both of its faces, all interior nodes of the other
-// two axes.
+// two axes.  Bound by memory latency; the loads come before the stores: with
+// the farther ghost loaded behind a store the three launches took 43 us on
+// 384x96x96 cells (both parts of a two-float current, in L2; 65 from DRAM),
+// against 19 (24).
 template <typename T, int AX>
 __global__ void k_jfold_axis(T* j0, T* j1, Geo g) {
   const int nx = g.ix2 - g.ix1 + 1, ny = g.jy2 - g.jy1 + 1, nz = g.kz2 - g.kz1 + 1;
@@ -210,18 +213,15 @@ __global__ void k_jfold_axis(T* j0, T* j1, Geo g) {
   const int q = blockIdx.y;
   T* c = (q < g.nc ? j0 + g.ncell * q : j1 + g.ncell * (q - g.nc)) + goff(g, i, j, k);
   const long long s = (AX == 0) ? 1 : (AX == 1) ? g.n1p : (long long)g.n1p * g.n2p, d = hi ? s : -s;
-  const T a = c[0], b = c[d];
+  const bool two = hi || AX == 1;
+  const T a = c[0], b = c[d], e = two ? c[2 * d] : (T)0;
+  c[0] = two ? a + b + e : a + b;
   c[d] = (T)0;
-  if (hi || AX == 1) {
-    c[0] = a + b + c[2 * d];
-    c[2 * d] = (T)0;
-  } else {
-    c[0] = a + b;
-  }
+  if (two) c[2 * d] = (T)0;
 }
 // j1: the compensation part of a two-float current, or null.  2D in one sweep
-// (4 us against 8: launches are what counts); in 3D one launch per axis: the
-// one sweep took 60 us on 384x96x96 cells, the axes' launches 5 each.
+// (4 us against 8: launches are what counts), 3D in one launch per axis (the
+// one sweep takes 42 us where these take 19).
 template <typename T>
 void jfold_t(T* j0, T* j1, const Geo& g, cudaStream_t st) {
   const int nq = g.nc * (j1 ? 2 : 1);
