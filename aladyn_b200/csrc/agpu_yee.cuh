@@ -166,24 +166,40 @@ __device__ __forceinline__ void jfold_node(T* j0, T* j1, const Geo& g, int q, in
       k = hi ? g.kz2 : g.kz1;
     }
     T* c = (q < g.nc ? j0 + g.ncell * q : j1 + g.ncell * (q - g.nc)) + goff(g, i, j, k);
+    // All loads before the first store: a load behind a store to a line near
+    // it waits for that store (a 24-run 2D scan of 10 steps 11.7 ms with the
+    // loads in between, 11.2 so).
+    const bool xl = i == g.ix1, xh = i == g.ix2, yl = j == g.jy1, yh = j == g.jy2;
+    const bool zl = g.ndim == 3 && k == g.kz1, zh = g.ndim == 3 && k == g.kz2;
+    const T o = (T)0;
     T v = *c;
+    const T xl1 = xl ? c[-1] : o, xh1 = xh ? c[1] : o, xh2 = xh ? c[2] : o;
+    const T yl1 = yl ? c[-sy] : o, yl2 = yl ? c[-2 * sy] : o, yh1 = yh ? c[sy] : o, yh2 = yh ? c[2 * sy] : o;
+    const T zl1 = zl ? c[-sz] : o, zh1 = zh ? c[sz] : o, zh2 = zh ? c[2 * sz] : o;
     // the nearer, then the farther ghost node along one direction
-    auto two = [&](long long d) {
-      v = v + c[d] + c[2 * d];
-      c[d] = (T)0;
-      c[2 * d] = (T)0;
-    };
-    auto one = [&](long long d) {
-      v = v + c[d];
-      c[d] = (T)0;
-    };
-    if (i == g.ix1) one(-1);
-    if (i == g.ix2) two(1);
-    if (j == g.jy1) two(-sy);
-    if (j == g.jy2) two(sy);
-    if (g.ndim == 3) {
-      if (k == g.kz1) one(-sz);
-      if (k == g.kz2) two(sz);
+    if (xl) {
+      v = v + xl1;
+      c[-1] = o;
+    }
+    if (xh) {
+      v = v + xh1 + xh2;
+      c[1] = c[2] = o;
+    }
+    if (yl) {
+      v = v + yl1 + yl2;
+      c[-sy] = c[-2 * sy] = o;
+    }
+    if (yh) {
+      v = v + yh1 + yh2;
+      c[sy] = c[2 * sy] = o;
+    }
+    if (zl) {
+      v = v + zl1;
+      c[-sz] = o;
+    }
+    if (zh) {
+      v = v + zh1 + zh2;
+      c[sz] = c[2 * sz] = o;
     }
     *c = v;
   }
@@ -220,8 +236,8 @@ __global__ void k_jfold_axis(T* j0, T* j1, Geo g) {
   if (two) c[2 * d] = (T)0;
 }
 // j1: the compensation part of a two-float current, or null.  2D in one sweep
-// (4 us against 8: launches are what counts), 3D in one launch per axis (the
-// one sweep takes 42 us where these take 19).
+// (4 us against 8: launches are what counts), 3D in one launch per axis (20 us
+// on 384x96x96 cells, 24 from DRAM; the one sweep 23 and 36).
 template <typename T>
 void jfold_t(T* j0, T* j1, const Geo& g, cudaStream_t st) {
   const int nq = g.nc * (j1 ? 2 : 1);
