@@ -85,8 +85,6 @@ __global__ void k_env_grad(double* av, Geo g, double dxi, double dyi, double dzi
   }
 }
 
-__device__ __forceinline__ bool in_stencil(int lo, int n) { return lo >= 1 && lo + 2 <= n; }
-
 // set_env_acc (src/particles/grid_part_connect.f90:414-615) ->
 // lpf_env_momenta (src/dynamics/boris_push.f90:170-223) ->
 // set_env_density (grid_part_connect.f90:884-952), per particle: the qqh

@@ -233,6 +233,12 @@ __global__ void __launch_bounds__(CAcc<NDIM>::NT, (NDIM == 3) ? 1 : 2) k_env_acc
         const int fx = i + 1 - i0t;
         if ((unsigned)fx >= (unsigned)C::TX || j + 1 - j0t != wy || (NDIM == 3 && k + 1 - k0t != wz)) {
           raise_err(a.err, AGPU_EBIT_INDEX);  // not binned in this row
+        } else if (!in_stencil(i, g.n1p) || !in_stencil(ih, g.n1p) || !in_stencil(j, g.n2p) || !in_stencil(jh, g.n2p) ||
+                   (NDIM == 3 && (!in_stencil(k, g.n3p) || !in_stencil(kh, g.n3p)))) {
+          // the last tiles reach beyond the array: a record out there (only
+          // the host can put one) is not gathered or deposited; the position
+          // step drops it
+          raise_err(a.err, AGPU_EBIT_INDEX);
         } else {
           const int li = fx + 1, lj = wy + 1, lk = (NDIM == 3) ? wz + 1 : 0;
           const int hi = li + ih - i, hj = lj + jh - j, hk = (NDIM == 3) ? lk + kh - k : 0;

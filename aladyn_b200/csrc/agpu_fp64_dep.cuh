@@ -53,6 +53,8 @@ __device__ __forceinline__ void qqh64(double xp, double ax[3], double axh[3], in
   *ix = i - 1;
   *ihx = ih - 1;
 }
+// A three-node stencil from node lo on lies in an axis of n nodes.
+__device__ __forceinline__ bool in_stencil(int lo, int n) { return lo >= 1 && lo + 2 <= n; }
 
 // ============================================================================
 // Esirkepov deposit of one move (grid_part_connect.f90:956-1334) with FP64

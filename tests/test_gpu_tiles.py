@@ -10,10 +10,10 @@ either sign in another order, each rounded to 2^-53 of at most the largest
 import numpy as np
 import pytest
 
-from aladyn_b200.abi import AGPU_FP32_SPLIT, AGPU_FP64
+from aladyn_b200.abi import AGPU_EBIT_INDEX, AGPU_FP32_SPLIT, AGPU_FP64
 from aladyn_b200.sim import PicDevice, pack_slot
 from oracle.oracle import Oracle
-from tests.helpers import laser_fields, small_case
+from tests.helpers import laser_fields, small_case, sort_records
 
 pytestmark = pytest.mark.gpu
 
@@ -121,3 +121,41 @@ def test_env_tile_steps(ndim, nx, ny, nz, n, how, pmax):
     for c in range(2 * ndim):
         x, y = np.sort(a[:, c]), np.sort(b[:, c])
         assert np.abs(x - y).max() <= 1e-12 * np.abs(y).max(), c
+
+
+@pytest.mark.parametrize("ndim,nx,ny,nz", [(2, 33, 5, 1), (3, 33, 4, 4)])
+def test_env_records_beyond_the_array(ndim, nx, ny, nz):
+    """The last tiles reach beyond the field array.  A record placed out
+    there is refused (index error), deposits nothing and is dropped, as in the
+    per-particle kernels of the deterministic mode; a record outside the box
+    whose stencil lies in the array counts.  Grids to 1e-12 (see above)."""
+    from tests.test_envelope import env_case, numpy_init, pulse
+    p, g, ep = env_case(ndim, nx=nx, ny=ny, nz=nz, cap=1000, w_sh=0)
+    env0 = numpy_init(p, pulse(p, a0=1.0, xc_frac=0.5, wx_frac=0.3, wy_frac=0.4))
+    rec = records(p, 300, "spread", 0.5)
+    n, d, lo = [nx, ny, nz][:ndim], [p.dx, p.dy, p.dz], [p.gxmin, p.gymin, p.gzmin]
+    top = [63.4, 7.4, 5.4]  # the tiles' last nodes
+    k = 0
+    for a in range(ndim):
+        for far in (n[a] + 0.7, n[a] + 1.7, top[a]):  # above the box: within the array, beyond it, at the tiles' end
+            rec[k, a] = lo[a] + far * d[a]
+            k += 1
+    for a in range(ndim):
+        rec[k, a] = lo[a] + top[a] * d[a]
+    rec[:, 2 * ndim] = pack_slot(np.full(300, -1), np.zeros(300), np.full(300, 0.05, np.float32))
+    got = []
+    for det in (False, True):
+        dev = PicDevice(p)
+        dev.env_enable(ep)
+        dev.set_deterministic(det)
+        dev.set_envelope(env0)
+        dev.set_fields(0.02 * laser_fields(p))
+        dev.set_species(0, rec)
+        out = dev.env_run(p.dt, 1)
+        assert out.error_bits & AGPU_EBIT_INDEX
+        got.append((dev.get_envelope(), dev.get_env_source(), dev.get_fields(), dev.get_currents(),
+                    sort_records(dev.get_species(0))))
+        assert out.np[0] == got[-1][4].shape[0]
+        dev.close()
+    for a, b in zip(*got):
+        assert a.shape == b.shape and np.abs(a - b).max() <= 1e-12 * np.abs(b).max()
