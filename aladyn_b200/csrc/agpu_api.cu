@@ -1576,6 +1576,8 @@ int agpu_step(agpu_handle* h, int32_t iter, double t, int32_t initial_time, agpu
     out->error_bits = h->error_bits;
   }
   CK(cudaGraphLaunch(h->gexec, h->st));
+  for (int ic = 0; ic < p.nsp_run; ++ic)  // every one that has records is tiled: its counts are on the device
+    if (h->np[ic] > 0) h->stale[ic] = true;
   h->timers.launches_total += h->g_launches;
   h->timers.launches_push_deposit += h->g_push;
   h->timers.launches_yee += h->g_yee;

@@ -1,0 +1,47 @@
+"""The counts a host reads: particles alive, pushed and removed, in the
+synchronous steps, with deferred counts and with replayed step graphs.
+Particles are bit-exact in the first FP64 step and to rounding after it, so
+counts are compared exactly."""
+import pytest
+
+from aladyn_b200.sim import PicDevice
+from tests.helpers import laser_fields, small_case
+from tests.test_gpu_tiles import records
+
+pytestmark = pytest.mark.gpu
+
+
+def _dev(cls, p, rec):
+    d = cls(p)
+    d.set_fields(laser_fields(p))
+    for ic in range(p.nsp_run):
+        d.set_species(ic, rec[ic::p.nsp_run])
+    return d
+
+
+def _step(d, p, it):
+    out = d.lp_run(it * p.dt, it, initial_time=(it == 0))
+    return out[1] if isinstance(out, tuple) else out
+
+
+@pytest.mark.parametrize("graphs", [False, True])
+def test_deferred_counts_between_steps(graphs):
+    """Diagnostics after every step while particles leave the box: the count,
+    the sums and the pushes are those of synchronous steps, whether a step is
+    launched, captured or replayed."""
+    p = small_case(2, cap=30000, w_sh=0)
+    rec = records(p, 20000, "spread", 5.0)
+    a, b = _dev(PicDevice, p, rec), _dev(PicDevice, p, rec)
+    b.set_deferred_counts(True)
+    b.set_step_graphs(graphs)
+    last = 20000
+    for it in range(8):
+        oa = _step(a, p, it)
+        _step(b, p, it)
+        da, db = a.diag(), b.diag()
+        assert oa.np[0] == da.np[0] < last
+        last = da.np[0]
+        assert db.np[0] == da.np[0], it
+        assert abs(db.kin_energy[0] - da.kin_energy[0]) <= 1e-9 * da.kin_energy[0]
+    assert b.timers().pushes == a.timers().pushes
+    assert b.get_species(0).shape == a.get_species(0).shape
