@@ -1835,6 +1835,7 @@ static int step_impl(agpu_handle* h, int32_t iter, double t, int32_t initial_tim
     }
     if (int rc_ = settle_counts(h, out)) return rc_;
     if (int rc_ = drop_removed(h, ic)) return rc_;
+    h->binned[ic] = false;  // the particles move without new keys
     np = h->np[ic];
     CK(cudaMemsetAsync(&h->d_cnt->removed, 0, sizeof(unsigned long long), h->st));
     ph_begin(h, PH_PUSH);

@@ -2,10 +2,12 @@
 synchronous steps, with deferred counts and with replayed step graphs.
 Particles are bit-exact in the first FP64 step and to rounding after it, so
 counts are compared exactly."""
+import numpy as np
 import pytest
 
 from aladyn_b200.sim import PicDevice
-from tests.helpers import laser_fields, small_case
+from oracle.oracle import Oracle
+from tests.helpers import laser_fields, small_case, sort_records
 from tests.test_gpu_tiles import records
 
 pytestmark = pytest.mark.gpu
@@ -45,3 +47,17 @@ def test_deferred_counts_between_steps(graphs):
         assert abs(db.kin_energy[0] - da.kin_energy[0]) <= 1e-9 * da.kin_energy[0]
     assert b.timers().pushes == a.timers().pushes
     assert b.get_species(0).shape == a.get_species(0).shape
+
+
+def test_tiles_after_a_deterministic_step():
+    """A deterministic step moves the particles without new binning keys: the
+    tiled step after it bins them again."""
+    p = small_case(2, cap=30000, w_sh=0)
+    rec = records(p, 20000, "piled", 1.0)  # away from the faces: nothing is removed
+    dev, ora = _dev(PicDevice, p, rec), _dev(Oracle, p, rec)
+    for it in range(4):
+        dev.set_deterministic(it == 1)
+        out, oo = _step(dev, p, it), _step(ora, p, it)
+        assert out.error_bits == 0 and out.np[0] == oo.np[0] == 20000, it
+    a, b = sort_records(dev.get_species(0)), sort_records(ora.get_species(0))
+    assert np.abs(a[:, :4] - b[:, :4]).max() <= 1e-12 * np.abs(b[:, :4]).max()
