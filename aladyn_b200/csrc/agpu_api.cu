@@ -712,7 +712,7 @@ __global__ void k_shift_cells(int* cell, float* ox, long long n, int nshx, int n
 }
 
 // lp_window_xshift (src/dynamics/window.f90:276-347).
-int window_xshift(agpu_handle* h, int witr, int init_iter, agpu_step_out* out, bool alive) {
+int window_xshift(agpu_handle* h, int witr, int init_iter, agpu_step_out* out) {
   agpu_params& p = h->p;
   if (init_iter == 0) {
     h->xlapse = 0.0;
@@ -750,7 +750,9 @@ int window_xshift(agpu_handle* h, int witr, int init_iter, agpu_step_out* out, b
       CK(cudaGetLastError());
       h->timers.launches_total += 1;
     }
-    const long long before = alive && h->binned[ic] ? h->nalive[ic] : h->np[ic];
+    // records dropped by the pushes and still stored were counted there
+    if (int rc = refresh_counts(h)) return rc;
+    const long long before = h->binned[ic] ? h->nalive[ic] : h->np[ic];
     int rc = compact_species(h, ic, true);
     if (rc) return rc;
     out->removed[ic] += before - h->np[ic];
@@ -778,7 +780,7 @@ int window_xshift(agpu_handle* h, int witr, int init_iter, agpu_step_out* out, b
 // so every lattice column not yet injected) moves by -vb w_nst dt, the
 // particles at or left of gxmin (or past gxmax) are dropped along x only and
 // the columns that entered the box are injected.
-int comoving_coordinate(agpu_handle* h, double vb, int w_nst, int loc_it, agpu_step_out* out, bool alive) {
+int comoving_coordinate(agpu_handle* h, double vb, int w_nst, int loc_it, agpu_step_out* out) {
   agpu_params& p = h->p;
   if (loc_it == 0) return 0;
   const double dt_step = p.dt;
@@ -791,7 +793,9 @@ int comoving_coordinate(agpu_handle* h, double vb, int w_nst, int loc_it, agpu_s
   }
   for (int ic = 0; ic < p.nsp; ++ic) {
     if (h->np[ic] <= 0) continue;
-    const long long before = alive && h->binned[ic] ? h->nalive[ic] : h->np[ic];
+    // records dropped by the pushes and still stored were counted there
+    if (int rc = refresh_counts(h)) return rc;
+    const long long before = h->binned[ic] ? h->nalive[ic] : h->np[ic];
     int rc = compact_species(h, ic, true);
     if (rc) return rc;
     out->removed[ic] += before - h->np[ic];
@@ -821,19 +825,18 @@ long long xadv_launches(const agpu_handle* h) { return h->xadv.tmp ? 6 + 2LL * h
 
 // lp_run (src/dynamics/pic_evolve_in_time.f90 callers): the moving window
 // (w_speed > 0) or the comoving frame's coordinate step (w_speed < 0), every
-// w_sh steps inside [wi_time, wf_time); alive: records dropped in earlier
-// steps and still stored were counted then and are not counted as removed here
-int window_or_comoving(agpu_handle* h, int iter, double t, agpu_step_out* out, bool alive = false) {
+// w_sh steps inside [wi_time, wf_time)
+int window_or_comoving(agpu_handle* h, int iter, double t, agpu_step_out* out) {
   const agpu_params& p = h->p;
   if (p.w_sh <= 0 || !(t >= p.wi_time && t < p.wf_time) || iter % p.w_sh != 0) return 0;
   int rc = 0;
   if (p.w_speed > 0.0) {
     ph_begin(h, PH_WINDOW);
-    rc = window_xshift(h, p.w_sh, iter, out, alive);
+    rc = window_xshift(h, p.w_sh, iter, out);
     ph_end(h, PH_WINDOW);
   } else if (p.w_speed < 0.0) {
     ph_begin(h, PH_WINDOW);
-    rc = comoving_coordinate(h, -p.w_speed, p.w_sh, iter, out, alive);
+    rc = comoving_coordinate(h, -p.w_speed, p.w_sh, iter, out);
     ph_end(h, PH_WINDOW);
   }
   return rc;
@@ -2442,7 +2445,7 @@ int agpu_env_run(agpu_handle* h, int32_t iter, double t, agpu_step_out* out) {
   h->timers.launches_yee += 1;
   h->timers.launches_total += (p.ndim == 3 ? 3 : 1) + yee_launches(yee_coef(p), h->xadv.tmp != nullptr) + xadv_launches(h);
   h->timers.yee_cells += (long long)p.nx * p.ny * (p.ndim == 3 ? p.nz : 1);
-  if ((rc = window_or_comoving(h, iter, t, out, true))) return rc;
+  if ((rc = window_or_comoving(h, iter, t, out))) return rc;
   if (int rc_ = read_counters(h)) return rc_;
   for (int q = 0; q < 4; ++q) out->np[q] = h->binned[q] ? h->nalive[q] : h->np[q];
   out->xmn = p.xmn;

@@ -476,8 +476,8 @@ int agpu_set_deterministic(agpu_handle* h, int32_t on);
  * many steps ahead.  agpu_step_out.np and .error_bits then hold the values of
  * the last synchronisation point (a window shift, agpu_get_count,
  * agpu_get_species, agpu_diag, agpu_synchronize, or turning the mode off);
- * .removed is not filled.  Off by default (the reference's lp_run reports
- * the counts every step). */
+ * .removed holds a window shift's own drops only.  Off by default (the
+ * reference's lp_run reports the counts every step). */
 int agpu_set_deferred_counts(agpu_handle* h, int32_t on);
 /* Step graphs (on != 0, effective in deferred-count mode): a step between
  * window shifts (not the first step, no ionization, profiling off, every

@@ -5,6 +5,7 @@ counts are compared exactly."""
 import numpy as np
 import pytest
 
+from aladyn_b200.abi import AGPU_FP32_SPLIT, AGPU_FP64
 from aladyn_b200.sim import PicDevice
 from oracle.oracle import Oracle
 from tests.helpers import laser_fields, small_case, sort_records
@@ -61,3 +62,20 @@ def test_tiles_after_a_deterministic_step():
         assert out.error_bits == 0 and out.np[0] == oo.np[0] == 20000, it
     a, b = sort_records(dev.get_species(0)), sort_records(ora.get_species(0))
     assert np.abs(a[:, :4] - b[:, :4]).max() <= 1e-12 * np.abs(b[:, :4]).max()
+
+
+@pytest.mark.parametrize("precision", [AGPU_FP64, AGPU_FP32_SPLIT])
+def test_removed_counts_over_window_steps(precision):
+    """agpu_step_out.removed holds this step's drops, on window steps too:
+    np = np before - removed + injected, and the oracle's number (FP64)."""
+    p = small_case(2, cap=30000, w_sh=3, precision=precision)
+    rec = records(p, 20000, "spread", 5.0)
+    dev, ora = _dev(PicDevice, p, rec), _dev(Oracle, p, rec)
+    last, shifts = 20000, 0
+    for it in range(10):
+        out, oo = _step(dev, p, it), _step(ora, p, it)
+        assert out.np[0] == last - out.removed[0] + out.injected[0], it
+        if precision == AGPU_FP64:
+            assert out.removed[0] == oo.removed[0] > 0 and out.np[0] == oo.np[0], it
+        last, shifts = out.np[0], shifts + (out.nshx > 0)
+    assert shifts >= 2
