@@ -1694,6 +1694,7 @@ int agpu_x_step_many(agpu_handle** hs, int32_t n, agpu_x_ws* w) {
     m.yc = yee_coef(p);
     bds = bds && m.yc.se2 == 0.0;
     m.cursor = h->cursor;
+    m.scan_tmp = h->scan_tmp;
     m.pushed = &h->d_cnt->pushed;
     m.removed = &h->d_cnt->removed;
     m.fmax = &h->d_cnt->fmax;

@@ -18,6 +18,7 @@ struct MultiInst {
   float* ebf;                  // fields (written by the field phases)
   YeeC yc;
   int* cursor;                 // scatter cursors (nkeys + 1), set by the scan
+  int* scan_tmp;               // block sums of the scan (bin_scan_tmp_ints)
   unsigned long long* pushed;  // the instance's device push counter
   unsigned long long* removed;
   double* fmax;

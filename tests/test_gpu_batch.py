@@ -20,6 +20,8 @@ import pytest
 from aladyn_b200.abi import AGPU_FP32_SPLIT, AGPU_FP64
 from aladyn_b200.config import Grid, laser, make_params, n_over_nc_to_n0, plasma
 from aladyn_b200.sim import PicBatch, PicDevice
+from tests.helpers import grid_small, laser_fields
+from tests.test_gpu_tiles import records
 
 pytestmark = pytest.mark.gpu
 LAM0 = 0.8
@@ -106,5 +108,41 @@ def test_batch_matches_sequential_instances(precision, multi):
             fa, fb = got.get_fields(), ref.get_fields()
             l2 = math.sqrt(((fa - fb) ** 2).sum() / (fb ** 2).sum())
             assert l2 < 1e-4
+        ref.close()
+    batch.close()
+
+
+def _load(dev, p, n, seed):
+    dev.set_fields(laser_fields(p))
+    dev.set_species(0, records(p, n, "spread", 1.0, seed=seed))
+
+
+# grids of a batch, its x differences (der_ord) in turn, launches of a
+# multi-instance step
+FORMS = [([(3, 160, 64, 64), (3, 64, 9, 5)], [2], 9)]  # 221952 and 2304 keys: the first beyond the one-launch scan
+
+
+@pytest.mark.parametrize("grids,orders,launches", FORMS)
+def test_batch_forms(grids, orders, launches):
+    """Split-form batches against the instances stepped one by one.  Both sum
+    the currents in FP32, in other orders: a few 2^-24 of a step's current, so
+    the fields agree to 1e-5 of their norm after three steps."""
+    n, steps = 40000, 4
+    ps = [make_params(grid_small(*g), precision=AGPU_FP32_SPLIT, capacity=(n + 16, 0, 0, 0), w_sh=0,
+                      der_ord=orders[i % len(orders)]) for i, g in enumerate(grids)]
+    batch = PicBatch(ps)
+    for i, (d, p) in enumerate(zip(batch.instances, ps)):
+        _load(d, p, n, i)
+    assert batch.run(steps, nthreads=2) == [0] * len(ps)
+    assert batch.launches() == launches * (steps - 1)  # the first steps run instance by instance
+    for i, (d, p) in enumerate(zip(batch.instances, ps)):
+        ref = PicDevice(p)
+        _load(ref, p, n, i)
+        for it in range(steps):
+            ref.lp_run(it * p.dt, it, initial_time=(it == 0))
+        assert abs(d.count(0) - ref.count(0)) <= 2 and ref.count(0) < n
+        for f in ("get_fields", "get_currents"):
+            a, b = getattr(d, f)(), getattr(ref, f)()
+            assert np.linalg.norm(a - b) <= 1e-5 * np.linalg.norm(b), (i, f)
         ref.close()
     batch.close()
