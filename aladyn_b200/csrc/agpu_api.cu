@@ -132,12 +132,6 @@ struct agpu_handle {
   int* tstart[4] = {nullptr, nullptr, nullptr, nullptr};
   int* cursor = nullptr;
   int* scan_tmp = nullptr;
-  // FP64 staging of host transfers (grown up to STAGE_MAX doubles and kept:
-  // a device allocation and its release in every call took 2 to 8 ms beside
-  // steps of 0.1 to 2 ms); larger arrays pass through it in chunks, in order
-  // on the handle's stream
-  double* stage = nullptr;
-  long long stage_n = 0;
   bool binned[4] = {false, false, false, false};
   long long nalive[4] = {0, 0, 0, 0};  // np minus removed records still stored
   // deferred counts: tiled steps leave the alive counts and the error word
@@ -186,20 +180,21 @@ int dmalloc(void** p, size_t bytes) {
   return 0;
 }
 
-// The staging buffer, at least min(n, STAGE_MAX) doubles.
-constexpr long long STAGE_MAX = 1ll << 23;
-int stage_grow(agpu_handle* h, long long n) {
-  n = std::min(n, STAGE_MAX);
-  if (h->stage_n >= n) return 0;
-  if (h->stage) {
-    cudaStreamSynchronize(h->st);
-    cudaFree(h->stage);
-  }
-  h->stage = nullptr;
-  h->stage_n = 0;
-  if (dmalloc((void**)&h->stage, sizeof(double) * n)) return AGPU_E_NOMEM;
-  h->stage_n = n;
-  return 0;
+// FP64 staging of host transfers: the larger of the two buffers that hold
+// nothing between steps, the fused Yee step's output (every node is written
+// before it is read) and the compaction target (the split form's slot column
+// of it).  Arrays beyond it pass through in chunks, in order on the handle's
+// stream.  A device allocation and its release in every call took 2 to 8 ms
+// beside steps of 0.1 to 2 ms.
+struct Stage {
+  double* p;
+  long long n;  // doubles
+};
+Stage stage_of(const agpu_handle* h) {
+  const long long nf = h->g.ncell * h->g.nf;
+  const Stage grid = h->fp32 ? Stage{(double*)h->ebf32_alt, nf / 2} : Stage{h->ebf_alt, nf};
+  const Stage part = h->fp32 ? Stage{(double*)h->sptmp.slot, h->capmax} : Stage{h->tmp, h->capmax * h->ndv};
+  return grid.n > part.n ? grid : part;
 }
 
 // Comoving frame (w_speed < 0: vbeam = -w_speed, set_init_param.f90:239-245):
@@ -280,7 +275,6 @@ int free_all(agpu_handle* h) {
   }
   cudaFree(h->cursor);
   cudaFree(h->scan_tmp);
-  cudaFree(h->stage);
   cudaFree(h->env);
   cudaFree(h->env_av);
   cudaFree(h->env_den);
@@ -1206,11 +1200,11 @@ int agpu_set_fields(agpu_handle* h, const double* ebf, int32_t n1p, int32_t n2p,
   if (!h->fp32) {
     CK(cudaMemcpyAsync(h->ebf, ebf, sizeof(double) * n, cudaMemcpyHostToDevice, h->st));
   } else {
-    if (int rc = stage_grow(h, (long long)n)) return rc;
-    for (size_t q = 0; q < n; q += STAGE_MAX) {
-      const size_t m = std::min(n - q, (size_t)STAGE_MAX);
-      CK(cudaMemcpyAsync(h->stage, ebf + q, sizeof(double) * m, cudaMemcpyHostToDevice, h->st));
-      f64_to_f32(h->stage, h->ebf32 + q, (long long)m, h->st, h->sms);
+    const Stage sg = stage_of(h);
+    for (size_t q = 0; q < n; q += sg.n) {
+      const size_t m = std::min(n - q, (size_t)sg.n);
+      CK(cudaMemcpyAsync(sg.p, ebf + q, sizeof(double) * m, cudaMemcpyHostToDevice, h->st));
+      f64_to_f32(sg.p, h->ebf32 + q, (long long)m, h->st, h->sms);
     }
     CK(cudaGetLastError());
   }
@@ -1227,11 +1221,11 @@ int agpu_get_fields(agpu_handle* h, double* ebf, int32_t n1p, int32_t n2p, int32
   if (!h->fp32) {
     CK(cudaMemcpyAsync(ebf, h->ebf, sizeof(double) * n, cudaMemcpyDeviceToHost, h->st));
   } else {
-    if (int rc = stage_grow(h, (long long)n)) return rc;
-    for (size_t q = 0; q < n; q += STAGE_MAX) {
-      const size_t m = std::min(n - q, (size_t)STAGE_MAX);
-      f32_to_f64(h->ebf32 + q, h->stage, (long long)m, h->st, h->sms);
-      CK(cudaMemcpyAsync(ebf + q, h->stage, sizeof(double) * m, cudaMemcpyDeviceToHost, h->st));
+    const Stage sg = stage_of(h);
+    for (size_t q = 0; q < n; q += sg.n) {
+      const size_t m = std::min(n - q, (size_t)sg.n);
+      f32_to_f64(h->ebf32 + q, sg.p, (long long)m, h->st, h->sms);
+      CK(cudaMemcpyAsync(ebf + q, sg.p, sizeof(double) * m, cudaMemcpyDeviceToHost, h->st));
     }
   }
   CK(cudaStreamSynchronize(h->st));
@@ -1245,15 +1239,15 @@ int agpu_get_currents(agpu_handle* h, double* jc, int32_t n1p, int32_t n2p, int3
   // curr = djc(i) * curr (curr_and_fields_util.f90:111-115), whole array,
   // scaled on the way out
   const size_t n = (size_t)g.ncell;
-  if (int rc = stage_grow(h, (long long)n)) return rc;
+  const Stage sg = stage_of(h);
   for (int c = 0; c < g.nc; ++c) {
     const double d = h->p.iform < 2 ? h->p.djc[c] : 1.0;
-    for (size_t q = 0; q < n; q += STAGE_MAX) {
-      const size_t m = std::min(n - q, (size_t)STAGE_MAX), o = n * c + q;
-      if (h->fp32) scaled_out(nullptr, h->jhi + o, h->jlo + o, h->stage, d, (long long)m, h->st, h->sms);
-      else scaled_out(h->jc + o, nullptr, nullptr, h->stage, d, (long long)m, h->st, h->sms);
+    for (size_t q = 0; q < n; q += sg.n) {
+      const size_t m = std::min(n - q, (size_t)sg.n), o = n * c + q;
+      if (h->fp32) scaled_out(nullptr, h->jhi + o, h->jlo + o, sg.p, d, (long long)m, h->st, h->sms);
+      else scaled_out(h->jc + o, nullptr, nullptr, sg.p, d, (long long)m, h->st, h->sms);
       CK(cudaGetLastError());
-      CK(cudaMemcpyAsync(jc + o, h->stage, sizeof(double) * m, cudaMemcpyDeviceToHost, h->st));
+      CK(cudaMemcpyAsync(jc + o, sg.p, sizeof(double) * m, cudaMemcpyDeviceToHost, h->st));
     }
   }
   CK(cudaStreamSynchronize(h->st));
@@ -1293,13 +1287,13 @@ int agpu_set_species(agpu_handle* h, int32_t ic, const double* part, int64_t ld,
       CK(cudaMemcpy2DAsync(h->part[ic], sizeof(double) * h->cap[ic], part, sizeof(double) * ld, sizeof(double) * np, ndv,
                            cudaMemcpyHostToDevice, h->st));
   } else if (np > 0) {
-    if (int rc = stage_grow(h, np * ndv)) return rc;
-    const long long chunk = STAGE_MAX / ndv;
+    const Stage sg = stage_of(h);
+    const long long chunk = sg.n / ndv;
     for (long long q = 0; q < np; q += chunk) {
       const long long m = std::min<long long>(np - q, chunk);
-      CK(cudaMemcpy2DAsync(h->stage, sizeof(double) * m, part + q, sizeof(double) * ld, sizeof(double) * m, ndv,
+      CK(cudaMemcpy2DAsync(sg.p, sizeof(double) * m, part + q, sizeof(double) * ld, sizeof(double) * m, ndv,
                            cudaMemcpyHostToDevice, h->st));
-      rec_to_split(h->stage, m, m, h->sp[ic].view(), q, h->g, h->p.xmn, h->p.ymn, h->p.zmn, h->p.dx_inv, h->p.dy_inv,
+      rec_to_split(sg.p, m, m, h->sp[ic].view(), q, h->g, h->p.xmn, h->p.ymn, h->p.zmn, h->p.dx_inv, h->p.dy_inv,
                    h->p.dz_inv, h->st, h->sms);
       CK(cudaGetLastError());
     }
@@ -1327,8 +1321,8 @@ int agpu_get_species(agpu_handle* h, int32_t ic, double* part, int64_t ld, int64
     CK(cudaMemcpy2DAsync(part, sizeof(double) * ld, h->part[ic], sizeof(double) * h->cap[ic], sizeof(double) * n, ndv,
                          cudaMemcpyDeviceToHost, h->st));
   } else {
-    if (int rc = stage_grow(h, n * ndv)) return rc;
-    const long long chunk = STAGE_MAX / ndv;
+    const Stage sg = stage_of(h);
+    const long long chunk = sg.n / ndv;
     for (long long q = 0; q < n; q += chunk) {
       const long long m = std::min(n - q, chunk);
       Part32View v = h->sp[ic].view();
@@ -1342,9 +1336,9 @@ int agpu_get_species(agpu_handle* h, int32_t ic, double* part, int64_t ld, int64
         v.pz += q;
       }
       v.slot += q;
-      split_to_rec(v, m, h->stage, m, h->g, h->p.xmn, h->p.ymn, h->p.zmn, h->p.dx, h->p.dy, h->p.dz, h->st, h->sms);
+      split_to_rec(v, m, sg.p, m, h->g, h->p.xmn, h->p.ymn, h->p.zmn, h->p.dx, h->p.dy, h->p.dz, h->st, h->sms);
       CK(cudaGetLastError());
-      CK(cudaMemcpy2DAsync(part + q, sizeof(double) * ld, h->stage, sizeof(double) * m, sizeof(double) * m, ndv,
+      CK(cudaMemcpy2DAsync(part + q, sizeof(double) * ld, sg.p, sizeof(double) * m, sizeof(double) * m, ndv,
                            cudaMemcpyDeviceToHost, h->st));
     }
   }
@@ -2197,13 +2191,13 @@ int agpu_window_inject(agpu_handle* h, int32_t ic, const double* part, int64_t l
     CK(cudaMemcpy2DAsync(h->part[ic] + h->np[ic], sizeof(double) * h->cap[ic], part, sizeof(double) * ld, sizeof(double) * n,
                          ndv, cudaMemcpyHostToDevice, h->st));
   } else {
-    if (int rc = stage_grow(h, n * ndv)) return rc;
-    const long long chunk = STAGE_MAX / ndv;
+    const Stage sg = stage_of(h);
+    const long long chunk = sg.n / ndv;
     for (long long q0 = 0; q0 < n; q0 += chunk) {
       const long long m = std::min<long long>(n - q0, chunk);
-      CK(cudaMemcpy2DAsync(h->stage, sizeof(double) * m, part + q0, sizeof(double) * ld, sizeof(double) * m, ndv,
+      CK(cudaMemcpy2DAsync(sg.p, sizeof(double) * m, part + q0, sizeof(double) * ld, sizeof(double) * m, ndv,
                            cudaMemcpyHostToDevice, h->st));
-      rec_to_split(h->stage, m, m, h->sp[ic].view(), h->np[ic] + q0, h->g, h->p.xmn, h->p.ymn, h->p.zmn, h->p.dx_inv,
+      rec_to_split(sg.p, m, m, h->sp[ic].view(), h->np[ic] + q0, h->g, h->p.xmn, h->p.ymn, h->p.zmn, h->p.dx_inv,
                    h->p.dy_inv, h->p.dz_inv, h->st, h->sms);
       CK(cudaGetLastError());
     }
