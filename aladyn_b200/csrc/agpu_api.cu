@@ -1770,23 +1770,18 @@ static int halo_call(agpu_handle* h, int point, int ic) {
 }
 static int yee_halo(void* ctx, int point) { return halo_call((agpu_handle*)ctx, point, -1); }
 
-static int step_impl(agpu_handle* h, int32_t iter, double t, int32_t initial_time, agpu_step_out* out) {
-  if (!h) return AGPU_E_ARG;
+static int step_body(agpu_handle* h, int32_t iter, double t, int32_t initial_time, agpu_step_out* out) {
   agpu_step_out dummy;
   if (!out) out = &dummy;
   std::memset(out, 0, sizeof(*out));
   out->ion_field_max = -1.0;
   agpu_params& p = h->p;
   int rc = 0;
-  for (int ic = 0; ic < 4; ++ic) h->pend[ic] = -1;
-  if (h->defer) {
-    // the error word and the push count keep accumulating on the device (the
-    // untiled push and the ionization clear their own counters)
-    if (p.ionz_lev > 0)
-      if (int rc_ = refresh_counts(h)) return rc_;
-  } else {
-    CK(cudaMemsetAsync(h->d_cnt, 0, sizeof(Counters), h->st));
-  }
+  // deferred: the error word and the push count keep accumulating on the
+  // device (the untiled push and the ionization clear their own counters)
+  if (!h->defer || p.ionz_lev > 0)
+    if (int rc_ = refresh_counts(h)) return rc_;
+  if (!h->defer) CK(cudaMemsetAsync(h->d_cnt, 0, sizeof(Counters), h->st));
   // pfields_prepare -> field_xyzbd; with one tiled species, binned by the
   // step before, jc = 0 and its histogram reset in the same launch
   const bool pre = p.nsp_run == 1 && p.ionz_lev == 0 && h->np[0] > 0 && h->binned[0] && tiled(h, 0);
@@ -1981,6 +1976,18 @@ static int step_impl(agpu_handle* h, int32_t iter, double t, int32_t initial_tim
   out->error_bits = h->error_bits;
   if (h->error_bits & AGPU_EBIT_CAPACITY) return AGPU_E_CAPACITY;
   return 0;
+}
+
+static int step_impl(agpu_handle* h, int32_t iter, double t, int32_t initial_time, agpu_step_out* out) {
+  const int rc = step_body(h, iter, t, initial_time, out);
+  // a step that ended early: the counts of its pushes are read at the next
+  // synchronisation point
+  for (int ic = 0; ic < 4; ++ic)
+    if (h->pend[ic] >= 0) {
+      h->stale[ic] = true;
+      h->pend[ic] = -1;
+    }
+  return rc;
 }
 
 // ---- stretched transverse grids ------------------------------------------------

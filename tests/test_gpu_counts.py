@@ -2,6 +2,10 @@
 synchronous steps, with deferred counts and with replayed step graphs.
 Particles are bit-exact in the first FP64 step and to rounding after it, so
 counts are compared exactly."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -79,3 +83,53 @@ def test_removed_counts_over_window_steps(precision):
             assert out.removed[0] == oo.removed[0] > 0 and out.np[0] == oo.np[0], it
         last, shifts = out.np[0], shifts + (out.nshx > 0)
     assert shifts >= 2
+
+
+# cudaMemcpyAsync with one device-to-host copy that fails on the host, when armed
+SHIM = """
+#include <dlfcn.h>
+#include <stddef.h>
+int armed = 0;
+int cudaMemcpyAsync(void* d, const void* s, size_t n, int kind, void* st) {
+  static int (*real)(void*, const void*, size_t, int, void*);
+  if (!real) real = (int (*)(void*, const void*, size_t, int, void*))dlsym(
+      dlopen("libcudart.so.12", RTLD_LAZY | RTLD_NOLOAD), "cudaMemcpyAsync");
+  if (armed && kind == 2) { armed = 0; return 2; }
+  return real(d, s, n, kind, st);
+}
+"""
+FAILED_READ = """
+import ctypes, sys
+from aladyn_b200.sim import PicDevice
+from tests.helpers import small_case
+from tests.test_gpu_counts import _dev, _step
+from tests.test_gpu_tiles import records
+armed = ctypes.c_int.in_dll(ctypes.CDLL(sys.argv[1]), "armed")
+p = small_case(2, cap=30000, w_sh=0)
+rec = records(p, 20000, "spread", 5.0)
+a, b = _dev(PicDevice, p, rec), _dev(PicDevice, p, rec)
+for it in range(4):
+    n = _step(a, p, it).np[0]
+    armed.value = it == 1
+    try:
+        _step(b, p, it)
+        assert it != 1
+    except RuntimeError:
+        assert it == 1 and armed.value == 0
+        assert b.count(0) == n < 20000, (b.count(0), n)
+        assert b.diag().np[0] == n
+assert b.count(0) == a.count(0) and b.get_species(0).shape == a.get_species(0).shape
+print("counts ok")
+"""
+
+
+def test_counts_after_a_failed_read(tmp_path):
+    """A step whose read of the counts fails (a host-side fake of the copy)
+    returns an error; the counts are read at the next call."""
+    src, lib = tmp_path / "shim.c", tmp_path / "shim.so"
+    src.write_text(SHIM)
+    subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(lib), str(src), "-ldl"], check=True)
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", FAILED_READ, str(lib)], cwd=root, capture_output=True, text=True,
+                       env=dict(os.environ, LD_PRELOAD=str(lib)), timeout=300)
+    assert r.returncode == 0 and "counts ok" in r.stdout, r.stdout + r.stderr
