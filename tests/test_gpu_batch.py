@@ -119,7 +119,14 @@ def _load(dev, p, n, seed):
 
 # grids of a batch, its x differences (der_ord) in turn, launches of a
 # multi-instance step
-FORMS = [([(3, 160, 64, 64), (3, 64, 9, 5)], [2], 9)]  # 221952 and 2304 keys: the first beyond the one-launch scan
+FORMS = [
+    ([(3, 160, 64, 64), (3, 64, 9, 5)], [2], 9),  # 221952 and 2304 keys: the first beyond the one-launch scan
+    ([(3, 37, 11, 6), (3, 5, 4, 4), (3, 33, 7, 9)], [2], 8),  # 3D: fold, ghosts and sweeps
+    ([(3, 37, 11, 6), (3, 5, 4, 9)], [3], 11),  # the wide x difference: separate boundary sweeps
+    ([(2, 131, 37, 1), (2, 300, 130, 1)], [3], 11),
+    ([(3, 37, 11, 6), (3, 33, 7, 9), (3, 4, 5, 6)], [2, 3], 11),  # both differences in one batch
+    ([(2, 131, 37, 1), (2, 1200, 130, 1), (2, 4, 4, 1)], [3, 2], 11),  # 640, 20672 (six blocks of the scan) and 32 keys
+]
 
 
 @pytest.mark.parametrize("grids,orders,launches", FORMS)
@@ -127,7 +134,7 @@ def test_batch_forms(grids, orders, launches):
     """Split-form batches against the instances stepped one by one.  Both sum
     the currents in FP32, in other orders: a few 2^-24 of a step's current, so
     the fields agree to 1e-5 of their norm after three steps."""
-    n, steps = 40000, 4
+    n, steps = 20000, 4
     ps = [make_params(grid_small(*g), precision=AGPU_FP32_SPLIT, capacity=(n + 16, 0, 0, 0), w_sh=0,
                       der_ord=orders[i % len(orders)]) for i, g in enumerate(grids)]
     batch = PicBatch(ps)

@@ -10,7 +10,7 @@ import pytest
 from aladyn_b200.config import make_params
 from aladyn_b200.sim import PicDevice
 from oracle.oracle import Oracle
-from tests.helpers import grid_small, laser_fields, small_case
+from tests.helpers import grid_small, laser_fields, small_case, sort_records
 from tests.test_gpu_tiles import records
 
 pytestmark = pytest.mark.gpu
@@ -49,3 +49,25 @@ def test_key_scan_sizes(nx, ny):
         got.append(d.get_species(0))
     assert got[0].shape == got[1].shape
     assert np.array_equal(got[0].view(np.uint64), got[1].view(np.uint64))
+
+
+@pytest.mark.parametrize("der_ord", [2, 3])
+@pytest.mark.parametrize("ndim,nx,ny,nz", [(2, 4, 4, 1), (2, 131, 37, 1), (3, 4, 4, 4), (3, 37, 6, 5)])
+def test_tiled_steps_with_merged_setup(ndim, nx, ny, nz, der_ord):
+    """From the second step on a tiled FP64 species takes the set-up launch
+    (field ghosts, cleared currents, histogram) and the particles have only
+    to be binned by the step before.  The currents differ from the oracle's by
+    the order of their FP64 sums, 1e-12 of the largest value as in
+    test_gpu_tiles; three steps multiply that by less than ten."""
+    n = 2000
+    got = []
+    for cls in (PicDevice, Oracle):
+        p = make_params(grid_small(ndim, nx, ny, nz), capacity=(n + 16, 0, 0, 0), w_sh=0, der_ord=der_ord)
+        d = cls(p)
+        d.set_fields(laser_fields(p))
+        d.set_species(0, records(p, n, "spread", 1.0))
+        for it in range(4):
+            d.lp_run(it * p.dt, it, initial_time=(it == 0))
+        got.append((d.get_fields(), d.get_currents(), sort_records(d.get_species(0))))
+    for a, b in zip(*got):
+        assert a.shape == b.shape and np.abs(a - b).max() <= 1e-11 * np.abs(b).max()

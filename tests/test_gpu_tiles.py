@@ -105,12 +105,15 @@ def env_step(cls, p, ep, rec, ebf, env0, nsteps):
 def test_env_tile_steps(ndim, nx, ny, nz, n, how, pmax):
     """Three envelope steps (the binning of one step serves the next): the
     density and current sums reach every output, so 1e-12 of the largest
-    value (see above); the records are compared as sorted columns."""
+    value (see above).  The tiles keep the records in another order: whole
+    rows are compared, matched through each record's own weight."""
     from tests.test_envelope import env_case, numpy_init, pulse
     p, g, ep = env_case(ndim, nx=nx, ny=ny, nz=nz, der_ord=2, cap=n + 16, w_sh=10)
     env0 = numpy_init(p, pulse(p, a0=1.0, xc_frac=0.5, wx_frac=0.3, wy_frac=0.4))
     rec, ebf = records(p, n, how, pmax), 0.02 * laser_fields(p)
-    rec[:, 2 * ndim] = pack_slot(np.full(n, -1), np.zeros(n), np.full(n, 0.01 / max(n / 1000, 1), np.float32))
+    wgh = 0.01 / max(n / 1000, 1) * (1 + np.arange(n) / n)  # one weight a record, FP32 numbers apart
+    rec[:, 2 * ndim] = pack_slot(np.full(n, -1), np.zeros(n), wgh)
+    assert np.unique(rec[:, 2 * ndim].view(np.uint64)).size == n
     dev = env_step(PicDevice, p, ep, rec, ebf, env0, 3)
     ora = env_step(Oracle, p, ep, rec, ebf, env0, 3)
     for f in ("get_envelope", "get_env_source", "get_fields", "get_currents"):
@@ -118,9 +121,10 @@ def test_env_tile_steps(ndim, nx, ny, nz, n, how, pmax):
         assert np.abs(a - b).max() <= 1e-12 * np.abs(b).max(), f
     a, b = dev.get_species(0), ora.get_species(0)
     assert a.shape == b.shape
+    a, b = (q[np.argsort(q[:, 2 * ndim].view(np.uint64))] for q in (np.ascontiguousarray(a), np.ascontiguousarray(b)))
+    assert np.array_equal(a[:, 2 * ndim].view(np.uint64), b[:, 2 * ndim].view(np.uint64))
     for c in range(2 * ndim):
-        x, y = np.sort(a[:, c]), np.sort(b[:, c])
-        assert np.abs(x - y).max() <= 1e-12 * np.abs(y).max(), c
+        assert np.abs(a[:, c] - b[:, c]).max() <= 1e-12 * np.abs(b[:, c]).max(), c
 
 
 @pytest.mark.parametrize("ndim,nx,ny,nz", [(2, 33, 5, 1), (3, 33, 4, 4)])
