@@ -130,6 +130,7 @@ struct agpu_handle {
   int* perm[4] = {nullptr, nullptr, nullptr, nullptr};
   int* hist[4] = {nullptr, nullptr, nullptr, nullptr};
   int* tstart[4] = {nullptr, nullptr, nullptr, nullptr};
+  RowList rows[4] = {};  // dense rows of the FP64 form's binnings, behind tstart
   int* cursor = nullptr;
   int* scan_tmp = nullptr;
   bool binned[4] = {false, false, false, false};
@@ -493,6 +494,8 @@ bool tiled(const agpu_handle* h, int ic) {
 int rebin(agpu_handle* h, int ic) {
   const TileGeo& t = h->tg;
   CK(cudaMemsetAsync(h->hist[ic], 0, sizeof(int) * (t.nkeys + 1), h->st));
+  if (h->rows[ic].n)  // the list of a binning that no push has used
+    CK(cudaMemsetAsync(h->rows[ic].n, 0, sizeof(unsigned int) * 2, h->st));
   if (h->fp32)
     bin_keys_split(h->sp[ic].cell, h->sp[ic].ox, h->sp[ic].oy, h->sp[ic].oz, h->np[ic], h->g, t, h->key[ic], h->hist[ic],
                    &h->d_cnt->err, h->st, h->sms);
@@ -500,7 +503,7 @@ int rebin(agpu_handle* h, int ic) {
     bin_keys_abs(h->part[ic], h->part[ic] + h->cap[ic], h->part[ic] + 2 * h->cap[ic], h->np[ic], h->g, t, h->p.xmn, h->p.ymn,
                  h->p.zmn, h->p.dx_inv, h->p.dy_inv, h->p.dz_inv, h->key[ic], h->hist[ic], &h->d_cnt->err, h->st, h->sms);
   const int nl = bin_finish(h->key[ic], h->np[ic], t, h->hist[ic], h->tstart[ic], h->cursor, h->perm[ic], h->scan_tmp,
-                            h->st, h->sms);
+                            h->rows[ic], h->st, h->sms);
   CK(cudaGetLastError());
   h->timers.launches_total += (h->np[ic] > 0 ? 1 : 0) + nl;  // keys, scan, scatter
   h->binned[ic] = true;
@@ -618,6 +621,8 @@ void tile_args64(const agpu_handle* h, int ic, int initial_time, TileArgs64& a) 
   a.vdt = comoving_vdt(p);
   a.initial = initial_time ? 1 : 0;
   a.err = &h->d_cnt->err;
+  a.rows = h->rows[ic];
+  a.extra = h->np[ic] > row_cap(h->np[ic], h->tg) ? 2 * h->sms : 0;
 }
 
 // Tiled gather + push + deposit of species ic (hist_done: the histogram is
@@ -674,7 +679,7 @@ int tiled_push(agpu_handle* h, int ic, int initial_time, bool hist_done) {
   if (!h->defer) h->timers.pushes += alive0;
   ph_begin(h, PH_SORT);
   const int nl = bin_finish(h->key[ic], h->np[ic], h->tg, h->hist[ic], h->tstart[ic], h->cursor, h->perm[ic], h->scan_tmp,
-                            h->st, h->sms);
+                            h->rows[ic], h->st, h->sms);
   CK(cudaGetLastError());
   h->timers.launches_total += nl;  // scan + scatter
   if (h->defer) {
@@ -1110,7 +1115,11 @@ int agpu_create(const agpu_params* params, agpu_handle** out) {
       rc |= dmalloc((void**)&h->key[ic], sizeof(int) * capmax);
       rc |= dmalloc((void**)&h->perm[ic], sizeof(int) * capmax);
       rc |= dmalloc((void**)&h->hist[ic], sizeof(int) * (h->tg.nkeys + 1));
-      rc |= dmalloc((void**)&h->tstart[ic], sizeof(int) * (h->tg.nkeys + 2));
+      rc |= dmalloc((void**)&h->tstart[ic], sizeof(int) * (h->fp32 ? h->tg.nkeys + 2 : tstart_ints(capmax, h->tg)));
+      if (!rc && !h->fp32) {
+        h->rows[ic] = row_list(h->tstart[ic], capmax, h->tg);
+        cudaMemsetAsync(h->rows[ic].n, 0, sizeof(unsigned int) * 4, h->st);
+      }
     }
     if (!rc) rc |= dmalloc((void**)&h->cursor, sizeof(int) * (h->tg.nkeys + 1));
     if (!rc) rc |= dmalloc((void**)&h->scan_tmp, sizeof(int) * bin_scan_tmp_ints(h->tg));
@@ -2418,7 +2427,7 @@ int agpu_env_run(agpu_handle* h, int32_t iter, double t, agpu_step_out* out) {
     // stay stored (key nkeys) until the next compaction
     ph_begin(h, PH_SORT);
     const int nl = bin_finish(h->key[ic], h->np[ic], h->tg, h->hist[ic], h->tstart[ic], h->cursor, h->perm[ic],
-                              h->scan_tmp, h->st, h->sms);
+                              h->scan_tmp, h->rows[ic], h->st, h->sms);
     CK(cudaGetLastError());
     h->timers.launches_total += 1 + nl;  // histogram reset, scan and scatter
     CK(cudaMemcpyAsync(&h->d_cnt->alive, h->tstart[ic] + h->tg.nkeys, sizeof(int), cudaMemcpyDeviceToDevice, h->st));

@@ -144,9 +144,33 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_sums(const int* hist, int
   d_scan_sums(hist, n, blockIdx.x, bsum);
 }
 
+// The thread's rows with more than cap records, listed (SCAN_ITEMS keys from
+// `base` on are whole rows; key n - 1 marks removed records).
+__device__ __forceinline__ void list_rows(const int h[SCAN_ITEMS], int base, int n, int nq, const RowList& rows, int cap) {
+  int c[4], nrow = 4;  // four rows of quadrants or two of octants
+#pragma unroll
+  for (int r = 0; r < 4; ++r) c[r] = h[4 * r] + h[4 * r + 1] + h[4 * r + 2] + h[4 * r + 3];
+  if (nq == 8) {
+    c[0] += c[1];
+    c[1] = c[2] + c[3];
+    nrow = 2;
+  }
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int row = base / nq + r;
+    if (r >= nrow || (row + 1) * nq > n - 1 || c[r] <= cap) continue;
+    const int items = (c[r] - cap + ROW_ITEM - 1) / ROW_ITEM;
+    const unsigned e = atomicAdd(&rows.n[0], (unsigned)items);
+    for (int q = 0; q < items && e + q < (unsigned)rows.size; ++q) {
+      rows.item[2 * (e + q)] = row;
+      rows.item[2 * (e + q) + 1] = q * ROW_ITEM;
+    }
+  }
+}
+
 // Block blk of the scan; before[0..nbefore) adds up to its first value.
 __device__ __forceinline__ void d_scan(const int* hist, int n, const int* before, int nbefore, int blk, int* start,
-                                       int* cursor) {
+                                       int* cursor, int nq = 0, const RowList* rows = nullptr, int cap = 0) {
   int v = 0, first, total;
   for (int e = threadIdx.x; e < nbefore; e += SCAN_THREADS) v += before[e];
   block_exclusive_sum(v, &first);
@@ -167,21 +191,26 @@ __device__ __forceinline__ void d_scan(const int* hist, int n, const int* before
     run += h[k];
     if (base + k == n - 1) start[n] = run;
   }
+  if (rows) {
+    if (blk == 0 && threadIdx.x == 0) rows->n[3] = (unsigned)cap;
+    list_rows(h, base, n, nq, *rows, cap);
+  }
 }
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan(const int* hist, int n, const int* bsum, int* start, int* cursor) {
-  if (bsum) d_scan(hist, n, bsum, blockIdx.x, blockIdx.x, start, cursor);
-  else d_scan(hist, n, hist, blockIdx.x * SCAN_BLOCK, blockIdx.x, start, cursor);
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan(const int* hist, int n, const int* bsum, int* start, int* cursor,
+                                                       int nq, RowList rows, int cap) {
+  const int blk = blockIdx.x;
+  d_scan(hist, n, bsum ? bsum : hist, bsum ? blk : blk * SCAN_BLOCK, blk, start, cursor, nq, rows.n ? &rows : nullptr, cap);
 }
 
 // hist has nkeys+1 bins (the last one: removed particles).  scan_tmp holds
 // bin_scan_tmp_ints(t) ints.  Returns the kernels launched.
 int bin_finish(const int* key, long long np, const TileGeo& t, const int* hist, int* start, int* cursor, int* perm,
-               int* scan_tmp, cudaStream_t st, int sms) {
+               int* scan_tmp, const RowList& rows, cudaStream_t st, int sms) {
   const int n = t.nkeys + 1;
   const int nb = (n + SCAN_BLOCK - 1) / SCAN_BLOCK;
   const bool one = n <= SCAN_ONE;
   if (!one) k_scan_sums<<<nb, SCAN_THREADS, 0, st>>>(hist, n, scan_tmp);
-  k_scan<<<nb, SCAN_THREADS, 0, st>>>(hist, n, one ? nullptr : scan_tmp, start, cursor);
+  k_scan<<<nb, SCAN_THREADS, 0, st>>>(hist, n, one ? nullptr : scan_tmp, start, cursor, t.nq, rows, row_cap(np, t));
   if (np > 0) k_perm_scatter<<<grid_for(np, 256, sms, 16), 256, 0, st>>>(key, np, cursor, perm);
   return (one ? 1 : 2) + (np > 0 ? 1 : 0);
 }

@@ -61,6 +61,37 @@ __device__ __forceinline__ void hist_add(int* hist, int key) {
   if ((threadIdx.x & 31) == leader) atomicAdd(&hist[key], __popc(peers));
 }
 
+// Dense rows of the FP64 tile kernels, which give a row of 32 nodes to one
+// warp.  A row's own warp takes its first `cap` records; the scan lists the
+// rest in items of ROW_ITEM records, which further CTAs of the tile kernels'
+// launches share out over all their warps.  A bunch a few cells wide lies in a
+// handful of rows, and with one warp a row a launch ran at the pace of the
+// fullest: 4e6 electrons of sigma (8, 1, 1) cells in a 192x96x96 box took
+// 171 ms an envelope step against 6.3 so (FP64 standard cycle 115 against
+// 5.4); sigma (25, 6, 6): 4.9 against 3.2 (5.0 against 2.8).
+struct RowList {
+  unsigned int* n;  // items listed, items taken, CTAs that found no more, cap; null: no list (split form)
+  int* item;        // (row, first record past the cap) pairs
+  int size;         // items the list holds
+};
+constexpr int ROW_ITEM = 4096;
+// Records of a row that stay with its warp: four times the mean of all rows
+// (evenly dense plasma needs no sharing out, and an item stages its tile's
+// fields again), at least four groups.
+AGPU_HD int row_cap(long long np, const TileGeo& t) {
+  const long long nrows = (long long)t.nkeys / t.nq, c = (4 * np / nrows + 127) / 128 * 128;
+  return c < 512 ? 512 : c > (1 << 30) ? (1 << 30) : (int)c;
+}
+// Items of rows with np records in all: a row beyond its cap (>= 512) lists
+// at most one item more than its records fill.
+AGPU_HD int row_list_size(long long np) { return (int)(np / ROW_ITEM + np / 512 + 1); }
+// The list behind a binning's key starts: ints for both.
+AGPU_HD size_t tstart_ints(long long np, const TileGeo& t) { return (size_t)t.nkeys + 2 + 4 + 2 * (size_t)row_list_size(np); }
+inline RowList row_list(int* tstart, long long np, const TileGeo& t) {
+  int* n = tstart + t.nkeys + 2;
+  return RowList{(unsigned int*)n, n + 4, row_list_size(np)};
+}
+
 // The next histogram's reset: bins zero, the dead bin seeded with the records
 // already dead (no tile visits them); with `pushed` set, the alive count of
 // this push (tstart[nkeys]) is added to it (the deferred-count mode keeps the
@@ -89,7 +120,7 @@ void bin_keys_abs(const double* x, const double* y, const double* z, long long n
                   unsigned int* err, cudaStream_t st, int sms);
 // Returns the number of kernels it launched.
 int bin_finish(const int* key, long long np, const TileGeo& t, const int* hist, int* start, int* cursor, int* perm,
-               int* scan_tmp, cudaStream_t st, int sms);
+               int* scan_tmp, const RowList& rows, cudaStream_t st, int sms);
 // ints of bin_finish's scan_tmp
 int bin_scan_tmp_ints(const TileGeo& t);
 long long perm_compact64(const int* perm, long long nalive, double* part, double* tmp, long long cap, int ndv, bool xbox,

@@ -171,8 +171,11 @@ __device__ __forceinline__ void density_full(const Geo& g, double* d, const doub
     }
 }
 
+// The records [c0, qend) of row `row` of the tiles (tx, ty, NZT zp ..) for the
+// warp.
 template <int NDIM>
-__global__ void __launch_bounds__(CAcc<NDIM>::NT, (NDIM == 3) ? 1 : 2) k_env_acc_tile(EnvTileArgs a) {
+__device__ __forceinline__ void acc_rows(const EnvTileArgs& a, const int tx, const int ty, const int zp, const int row,
+                                         int c0, const int qend) {
   using C = CAcc<NDIM>;
   constexpr int FX = C::FX, FY = C::FY, FV = C::FV, NE = C::NE, S = C::S, ND = C::ND, RMAX = C::RMAX;
   extern __shared__ double smd[];
@@ -184,17 +187,8 @@ __global__ void __launch_bounds__(CAcc<NDIM>::NT, (NDIM == 3) ? 1 : 2) k_env_acc
   unsigned char* idx = reinterpret_cast<unsigned char*>(smd + C::DOUBLES) + sizeof(int) * C::INTS + warp * (RMAX + 1) * 32;
   unsigned char* ord = idx + RMAX * 32;
 
-  const int b = blockIdx.x, plane = a.t.ntx * a.t.nty;
-  const int tx = b % a.t.ntx, ty = (b / a.t.ntx) % a.t.nty, zp = b / plane;
   const int i0t = 3 + tx * C::TX, j0t = 3 + ty * C::TY, k0t = (NDIM == 3) ? 3 + zp * C::TZ : 1;
-  const int wy = warp % C::TY, wz = warp / C::TY;
-  // the warp's row: tile, then row inside the tile
-  const int tz = zp * C::NZT + wz / C::T::TZ;
-  const bool on = tz < a.t.ntz;
-  const int krow = ((tx + a.t.ntx * (ty + a.t.nty * tz)) * C::T::NROW + wy + C::TY * (wz % C::T::TZ)) * C::T::NQ;
-  int c0 = on ? a.tstart[krow] : 0;
-  const int qend = on ? a.tstart[krow + C::T::NQ] : 0;
-  if (!__syncthreads_or(c0 < qend)) return;
+  const int wy = row % C::TY, wz = row / C::TY;
 
   stage64<C::NF, FX, FY, C::FZ, C::NROW>(sF, g, i0t - 2, j0t - 2, (NDIM == 3) ? k0t - 2 : 1, [&](int c) {
     return c < NE ? a.ebf + g.ncell * c : a.av + g.ncell * (c - NE);
@@ -465,20 +459,49 @@ __global__ void __launch_bounds__(CAcc<NDIM>::NT, (NDIM == 3) ? 1 : 2) k_env_acc
   }
 }
 
+// A CTA of NZT tiles, or one of the `extra` CTAs for the dense rows' items.
+template <int NDIM>
+__global__ void __launch_bounds__(CAcc<NDIM>::NT, (NDIM == 3) ? 1 : 2) k_env_acc_tile(EnvTileArgs a) {
+  using C = CAcc<NDIM>;
+  using T = typename C::T;
+  const int warp = threadIdx.x >> 5, b = blockIdx.x, plane = a.t.ntx * a.t.nty;
+  const int cap = a.extra ? (int)a.rows.n[3] : 0x7fffffff;
+  if (b < (int)gridDim.x - a.extra) {
+    const int zp = b / plane, tile = zp * C::NZT * plane + b % plane + warp / T::NROW * plane;
+    int c0 = 0, end = 0;
+    if (tile < a.t.ntiles) {  // the last CTA along z may have fewer tiles
+      const int* start = a.tstart + (tile * T::NROW + warp % T::NROW) * T::NQ;
+      c0 = start[0];
+      end = start[T::NQ];
+    }
+    if (!__syncthreads_or(c0 < end)) return;
+    acc_rows<NDIM>(a, b % a.t.ntx, (b / a.t.ntx) % a.t.nty, zp, warp, c0, end - c0 > cap ? c0 + cap : end);
+    return;
+  }
+  if (a.rows.n[0] == 0u) return;
+  for (int q; (q = next_item(a.rows)) >= 0;) {
+    const int row = a.rows.item[2 * q], t = row / T::NROW, tz = t / plane, seg = ROW_ITEM / C::NROW;
+    const int c0 = a.tstart[row * T::NQ] + cap + a.rows.item[2 * q + 1] + warp * seg;
+    acc_rows<NDIM>(a, t % a.t.ntx, (t / a.t.ntx) % a.t.nty, tz / C::NZT, tz % C::NZT * T::NROW + row % T::NROW, c0,
+                   min(a.tstart[(row + 1) * T::NQ], c0 + seg));
+  }
+  items_done(a.rows, a.extra, false);  // the position step takes the same items
+}
+
 template <int NDIM>
 void acc_t(const EnvTileArgs& a, cudaStream_t st) {
   using C = CAcc<NDIM>;
   auto k = k_env_acc_tile<NDIM>;
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::BYTES);
   const int nzp = (NDIM == 3) ? (a.t.ntz + C::NZT - 1) / C::NZT : 1;
-  k<<<a.t.ntx * a.t.nty * nzp, C::NT, C::BYTES, st>>>(a);
+  k<<<a.t.ntx * a.t.nty * nzp + a.extra, C::NT, C::BYTES, st>>>(a);
 }
 template <int NDIM>
 void pos_t(const EnvTileArgs& a, cudaStream_t st) {
   using C = C64<NDIM, PushEnv<NDIM>::NF, PushEnv<NDIM>::LO>;
   auto k = k_env_pos_tile<NDIM>;
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::BYTES);
-  k<<<a.t.ntiles, C::NT, C::BYTES, st>>>(a);
+  k<<<a.t.ntiles + a.extra, C::NT, C::BYTES, st>>>(a);
 }
 
 }  // namespace

@@ -54,6 +54,8 @@ struct TileArgs64 {
   double vdt;  // comoving frame: dt * vbeam subtracted from x after the push (0: off)
   int initial;
   unsigned int* err;
+  RowList rows;  // dense rows
+  int extra;     // CTAs after the tiles' that take the rows' items (0: no row can be dense)
 };
 
 // The envelope cycle's particle steps on the same tiles: the source scratch

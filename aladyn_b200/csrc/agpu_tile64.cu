@@ -225,7 +225,7 @@ void tile_push64_t(const TileArgs64& a, cudaStream_t st) {
   using C = C64<NDIM, Push64<NDIM>::NF, Push64<NDIM>::LO>;
   auto k = k64_tile<NDIM>;
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::BYTES);
-  k<<<a.t.ntiles, C::NT, C::BYTES, st>>>(a);
+  k<<<a.t.ntiles + a.extra, C::NT, C::BYTES, st>>>(a);
 }
 
 }  // namespace
