@@ -405,10 +405,10 @@ __device__ __forceinline__ void tile64_rows(const typename P::Args& a, const int
           const int in = node_d(a.dx_inv * (xn[0] - a.xmn), sn[0]), jn = node_d(a.dy_inv * (xn[1] - a.ymn), sn[1]);
           const int kn = (NDIM == 3) ? node_d(a.dz_inv * (xn[2] - a.zmn), sn[2]) : 0;
           const int ih = in - (i0t + fx) + 1, jh = jn - (j0t + fy) + 1, kh = (NDIM == 3) ? kn - (k0t + fz) + 1 : 1;
-          if (keep && ((unsigned)ih > 2u || (unsigned)jh > 2u || (unsigned)kh > 2u)) {
-            raise_err(a.err, AGPU_EBIT_INDEX);  // moved more than one cell: no window slot
-            keep = false;
-          }
+          // a move of more than one cell has no window slot: no current, the
+          // record stays (the comoving frame can move one by almost two)
+          const bool slots = (unsigned)ih <= 2u && (unsigned)jh <= 2u && (unsigned)kh <= 2u;
+          if (keep && !slots) raise_err(a.err, AGPU_EBIT_INDEX);
           const int oct = offset_octant((float)sn[0], (float)sn[1], (float)sn[2], NDIM);
           const int nkey = keep ? tile_key_c<TX, TY, TZ, C::NQ>(a.t, in, jn, (NDIM == 3) ? kn : 3, oct) : a.t.nkeys;
           a.key[p] = nkey;
@@ -416,7 +416,7 @@ __device__ __forceinline__ void tile64_rows(const typename P::Args& a, const int
           // histogram once per tile
           if ((unsigned)(nkey - kbase) < (unsigned)C::NSUB) atomicAdd(&sHist[nkey - kbase], 1);
           else hist_add(a.hist, nkey);
-          if (keep) {
+          if (keep && slots) {
             dep[e] = so[0];
             dep[S + e] = so[1];
             if (NDIM == 3) dep[2 * S + e] = so[2];

@@ -15,6 +15,7 @@ Tolerances:
 import numpy as np
 import pytest
 
+from aladyn_b200.abi import AGPU_EBIT_INDEX
 from aladyn_b200.sim import PicDevice
 from oracle.oracle import Oracle
 from tests.helpers import laser_fields, plasma_source
@@ -127,6 +128,63 @@ def test_env_run_atomic_close(ndim):
     assert a.shape == b.shape
     for c in range(2 * ndim):
         assert _relmax(np.sort(a[:, c]), np.sort(b[:, c])) <= 1e-12, c
+
+
+def _hot_pair(ndim, w_speed, temp):
+    """Device (tiles) and oracle with a window event every fourth step and a
+    plasma of momenta temp * normal."""
+    p, g, ep = env_case(ndim, cap=200000, w_sh=4)
+    p.w_speed = w_speed
+    pair, hot = [], None
+    for cls in (Oracle, PicDevice):
+        d = cls(p)
+        d.env_enable(ep)
+        d.set_envelope(numpy_init(p, pulse(p, a0=1.5, xc_frac=0.6, wx_frac=0.1, wy_frac=0.3)))
+        d.set_fields(0.02 * laser_fields(p))
+        d.set_plasma_source(plasma_source(p, x_start_frac=0.3))
+        d.load_plasma(0)
+        if hot is None:
+            hot = d.get_species(0)
+            hot[:, ndim:2 * ndim] = temp * np.random.default_rng(4).standard_normal((hot.shape[0], ndim))
+        d.set_species(0, hot)
+        pair.append(d)
+    return p, pair[1], pair[0]
+
+
+@pytest.mark.parametrize("ndim", [2, 3])
+@pytest.mark.parametrize("w_speed,temp", [(1.0, 2.0), (-0.9, 0.05)])
+def test_env_tiles_over_window_events(ndim, w_speed, temp):
+    """The tiled steps across window shifts (or the comoving frame's
+    coordinate steps): the compaction takes the records along the binning and
+    leaves out those dropped since, the injected columns are binned anew.
+    Counts of every step, then grids to 1e-11 after 13 steps (1e-12 after 8
+    without events)."""
+    p, dev, ora = _hot_pair(ndim, w_speed, temp)
+    events = removed = 0
+    for it in range(1, 14):
+        out = dev.env_run(it * p.dt, it)
+        rc, oo = ora.env_run(it * p.dt, it)
+        assert rc == 0 and out.error_bits == 0
+        assert (out.np[0], out.removed[0], out.injected[0]) == (oo.np[0], oo.removed[0], oo.injected[0]), it
+        events, removed = events + (out.injected[0] > 0), removed + out.removed[0]
+    assert events >= 2 and (removed > 20 or w_speed < 0)
+    for f in ("get_envelope", "get_env_source", "get_fields", "get_currents"):
+        assert _relmax(getattr(dev, f)(), getattr(ora, f)()) <= 1e-11, f
+
+
+@pytest.mark.parametrize("ndim", [2, 3])
+def test_env_tiles_moves_beyond_a_cell(ndim):
+    """The comoving frame moves a particle by up to dt (1 + vbeam): one that
+    changes node by two is reported (index error) and deposits nothing, but
+    stays, as in the deterministic mode and in the oracle."""
+    p, dev, ora = _hot_pair(ndim, -0.9, 1.0)
+    for it in range(1, 6):
+        out = dev.env_run(it * p.dt, it)
+        rc, oo = ora.env_run(it * p.dt, it)
+        assert out.error_bits == ora.error_bits() == AGPU_EBIT_INDEX
+        assert (out.np[0], out.removed[0]) == (oo.np[0], oo.removed[0]), it
+    for f in ("get_envelope", "get_env_source", "get_fields", "get_currents"):
+        assert _relmax(getattr(dev, f)(), getattr(ora, f)()) <= 1e-11, f
 
 
 def test_env_requires_enable_and_fp64():
