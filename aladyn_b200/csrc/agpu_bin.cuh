@@ -77,10 +77,15 @@ struct RowList {
 constexpr int ROW_ITEM = 4096;
 // Records of a row that stay with its warp: four times the mean of all rows
 // (evenly dense plasma needs no sharing out, and an item stages its tile's
-// fields again), at least four groups.
+// fields again), and what a warp gets through while the launch takes an eighth
+// of its time (0.3 us a record against 0.13 ns of the whole chip: np / 16384),
+// at least four groups.  Without the second, smooth bunches and ionized regions
+// of large runs were cut up for nothing: 512x256x256 cells with a bunch of
+// sigma (25, 6, 6) took 52.4 ms an envelope step against 49.9, 768x192x192 cells
+// with ionization 30.4 against 27.8 (49.6 and 27.6 with no sharing out at all).
 AGPU_HD int row_cap(long long np, const TileGeo& t) {
-  const long long nrows = (long long)t.nkeys / t.nq, c = (4 * np / nrows + 127) / 128 * 128;
-  return c < 512 ? 512 : c > (1 << 30) ? (1 << 30) : (int)c;
+  const long long nrows = (long long)t.nkeys / t.nq, mean4 = 4 * np / nrows, c = mean4 > np / 16384 ? mean4 : np / 16384;
+  return c < 512 ? 512 : c > (1 << 30) ? (1 << 30) : (int)((c + 127) / 128 * 128);
 }
 // Items of rows with np records in all: a row beyond its cap (>= 512) lists
 // at most one item more than its records fill.

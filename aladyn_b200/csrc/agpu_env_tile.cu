@@ -479,11 +479,10 @@ __global__ void __launch_bounds__(CAcc<NDIM>::NT, (NDIM == 3) ? 1 : 2) k_env_acc
     return;
   }
   if (a.rows.n[0] == 0u) return;
-  for (int q; (q = next_item(a.rows)) >= 0;) {
-    const int row = a.rows.item[2 * q], t = row / T::NROW, tz = t / plane, seg = ROW_ITEM / C::NROW;
-    const int c0 = a.tstart[row * T::NQ] + cap + a.rows.item[2 * q + 1] + warp * seg;
-    acc_rows<NDIM>(a, t % a.t.ntx, (t / a.t.ntx) % a.t.nty, tz / C::NZT, tz % C::NZT * T::NROW + row % T::NROW, c0,
-                   min(a.tstart[(row + 1) * T::NQ], c0 + seg));
+  for (int q, c0, end; (q = next_item(a.rows)) >= 0;) {
+    const int row = a.rows.item[2 * q], t = row / T::NROW, tz = t / plane;
+    item_records(a.rows, a.tstart, T::NQ, q, warp, C::NROW, c0, end);
+    acc_rows<NDIM>(a, t % a.t.ntx, (t / a.t.ntx) % a.t.nty, tz / C::NZT, tz % C::NZT * T::NROW + row % T::NROW, c0, end);
   }
   items_done(a.rows, a.extra, false);  // the position step takes the same items
 }

@@ -296,6 +296,14 @@ __device__ __forceinline__ int next_item(const RowList& rows) {
   __syncthreads();
   return s_item;
 }
+// Records [c0, end) of item q for one of nwarps warps, evenly in batches of 32.
+__device__ __forceinline__ void item_records(const RowList& rows, const int* tstart, int nq, int q, int warp, int nwarps,
+                                             int& c0, int& end) {
+  const int row = rows.item[2 * q], first = tstart[row * nq] + (int)rows.n[3] + rows.item[2 * q + 1];
+  const int n = min(ROW_ITEM, tstart[(row + 1) * nq] - first), seg = (n + 32 * nwarps - 1) / (32 * nwarps) * 32;
+  c0 = first + min(n, warp * seg);
+  end = min(first + n, c0 + seg);
+}
 // After a CTA's last item: the last of the launch's `extra` CTAs, none of
 // which reads the list any more, rewinds it, or empties it for the next scan.
 __device__ __forceinline__ void items_done(const RowList& rows, int extra, bool empty) {
@@ -551,10 +559,10 @@ __device__ __forceinline__ void tile64_step(const typename P::Args& a) {
     return;
   }
   if (a.rows.n[0] == 0u) return;  // nothing to take or to rewind
-  for (int q; (q = next_item(a.rows)) >= 0;) {
-    const int row = a.rows.item[2 * q], seg = ROW_ITEM / C::NROW;
-    const int c0 = a.tstart[row * C::NQ] + cap + a.rows.item[2 * q + 1] + warp * seg;
-    tile64_rows<NDIM, P>(a, row / C::NROW, row % C::NROW, c0, min(a.tstart[(row + 1) * C::NQ], c0 + seg));
+  for (int q, c0, end; (q = next_item(a.rows)) >= 0;) {
+    const int row = a.rows.item[2 * q];
+    item_records(a.rows, a.tstart, C::NQ, q, warp, C::NROW, c0, end);
+    tile64_rows<NDIM, P>(a, row / C::NROW, row % C::NROW, c0, end);
   }
   items_done(a.rows, a.extra, true);
 }
