@@ -184,8 +184,9 @@ int dmalloc(void** p, size_t bytes) {
 // FP64 staging of host transfers: the larger of the two buffers that hold
 // nothing between steps, the fused Yee step's output (every node is written
 // before it is read) and the compaction target (the split form's slot column
-// of it).  Arrays beyond it pass through in chunks, in order on the handle's
-// stream.  A device allocation and its release in every call took 2 to 8 ms
+// of it).  Larger arrays pass through in chunks, in order on the handle's
+// stream, of at most 64 MB, which stay in L2 between the conversion and the
+// copy.  A device allocation and its release in every call took 2 to 8 ms
 // beside steps of 0.1 to 2 ms.
 struct Stage {
   double* p;
@@ -195,7 +196,8 @@ Stage stage_of(const agpu_handle* h) {
   const long long nf = h->g.ncell * h->g.nf;
   const Stage grid = h->fp32 ? Stage{(double*)h->ebf32_alt, nf / 2} : Stage{h->ebf_alt, nf};
   const Stage part = h->fp32 ? Stage{(double*)h->sptmp.slot, h->capmax} : Stage{h->tmp, h->capmax * h->ndv};
-  return grid.n > part.n ? grid : part;
+  const Stage big = grid.n > part.n ? grid : part;
+  return Stage{big.p, std::min(big.n, 1ll << 23)};
 }
 
 // Comoving frame (w_speed < 0: vbeam = -w_speed, set_init_param.f90:239-245):
