@@ -41,7 +41,7 @@ struct Counters {
   int alive;  // particles in tiles after the last binning
   double fmax;
   unsigned long long pushed;  // deferred mode: particles pushed since the last refresh
-  int alive4[4];              // deferred mode: alive count per species at the refresh
+  int alive4[4];              // alive count per species after the step's pushes (deferred: at the refresh)
 };
 
 }  // namespace
@@ -135,12 +135,12 @@ struct agpu_handle {
   int* scan_tmp = nullptr;
   bool binned[4] = {false, false, false, false};
   long long nalive[4] = {0, 0, 0, 0};  // np minus removed records still stored
+  // alive counts of this step's tiled pushes still on their way to the host
+  // (pend[ic] = the count before the push, -1: none); settle_counts reads
+  // them with the step's one synchronisation
+  long long pend[4] = {-1, -1, -1, -1};
   // deferred counts: tiled steps leave the alive counts and the error word
   // on the device; refresh_counts reads them at the next synchronisation
-  // pend: alive counts of this step's tiled pushes still on their way to the
-  // host (pend[ic] = the count before the push, -1: none); settle_counts
-  // reads them with the step's one synchronisation
-  long long pend[4] = {-1, -1, -1, -1};
   bool defer = false;
   bool stale[4] = {false, false, false, false};
   // step graph (deferred mode): the launches of a step between window

@@ -11,7 +11,7 @@
 // come from shared memory and the atomics are per node.  The earlier
 // per-particle kernels (stencils from global memory, 27 and 81 atomics a
 // particle) took 1.88 and 2.15 ms for 7.1e6 particles (192x96x96 cells, 4 per
-// cell) against 1.29 and 1.01 ms now.  Compiled with -fmad=false; the
+// cell) against 1.27 and 1.03 ms now.  Compiled with -fmad=false; the
 // arithmetic up to the deposits keeps the reference's statement order.
 #include "agpu_env.h"
 #include "agpu_fp64_dep.cuh"

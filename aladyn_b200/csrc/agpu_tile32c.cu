@@ -89,8 +89,10 @@ size_t tile32c_smem(int ndim, int tx, int ty, int tz) {
 }
 
 // Two CTAs per SM in 3D: the staged fields and currents (101 KB) allow no
-// third, and the 80 registers that three would leave a thread spilled (a pass
-// of 10 steps on 256x96x96 cells 46.8 ms, 38.7 without spills).
+// third, and the 80 registers that three would leave a thread spilled.  Driven
+// 256x96x96 cells, a pass of 10 steps: 46.8 ms, 38.7 without spills; a step's
+// push on 512x128x128 cells 7.9 -> 7.6 ms, on 1024x256x256, mostly at rest,
+// 53.8 -> 54.5.  (96 registers, 60 B of spills: 40.0, 7.7 and 53.6.)
 template <int NDIM, int TX, int TY, int TZ>
 __global__ void __launch_bounds__(256, (NDIM == 3) ? 2 : 3) k32c_tile(TileArgs32 a) {
   constexpr int FX = TX + 4, FY = TY + 4, FZ = (NDIM == 3) ? TZ + 4 : 1;

@@ -236,8 +236,8 @@ __global__ void k_jfold_axis(T* j0, T* j1, Geo g) {
   if (two) c[2 * d] = (T)0;
 }
 // j1: the compensation part of a two-float current, or null.  2D in one sweep
-// (4 us against 8: launches are what counts), 3D in one launch per axis (20 us
-// on 384x96x96 cells, 24 from DRAM; the one sweep 23 and 36).
+// (4 us against 8: launches are what counts), 3D in one launch per axis (on
+// 384x96x96 cells the 19 us above, 24 from DRAM; the one sweep 23 and 36).
 template <typename T>
 void jfold_t(T* j0, T* j1, const Geo& g, cudaStream_t st) {
   const int nq = g.nc * (j1 ? 2 : 1);

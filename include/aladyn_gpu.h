@@ -201,7 +201,9 @@ typedef struct agpu_diag_out {
  * library attributes to each phase (particle records read+written, cells). */
 typedef struct agpu_timers {
   double ms_push_deposit;  /* fused gather + push + deposit                       */
-  double ms_yee;           /* Yee update incl. boundaries and current fold        */
+  double ms_yee;           /* Yee update incl. boundaries, current fold and the
+                              step's set-up launch (ghosts; with one tiled species
+                              the cleared currents and histogram too)          */
   double ms_sort;          /* particle tile sort / compaction                     */
   double ms_window;        /* window shift + injection                            */
   double ms_ionize;        /* ion field, ionization draws, electron append        */
@@ -488,8 +490,9 @@ int agpu_set_deferred_counts(agpu_handle* h, int32_t on);
  * grids; the work done is the same. */
 int agpu_set_step_graphs(agpu_handle* h, int32_t on);
 /* The leapfrog Yee update (with its Mur boundaries) as one z-streaming
- * kernel writing a second field array (on), or as the six separate sweeps
- * and face kernels (off, the default).  Same results (bit for bit in FP64);
+ * kernel writing a second field array (on), or as three sweeps that form
+ * their own boundary values (six kernels with the wide x difference or the
+ * comoving frame; off, the default).  Same results (bit for bit in FP64);
  * the fused kernel moves each field word once, but with one column tile and
  * a few planes per CTA it is latency bound and on a B200 it is slower than
  * the separate kernels in 3D (faster in 2D).  Step graphs use the separate
