@@ -5,8 +5,10 @@
 //   * cell_split inverts goff on random nodes of several grids;
 //   * tile_key / tile_key_c: the key packs (tile, row, octant) as
 //     tile * nsub + row * nq + octant, nodes outside the tiles map to nkeys,
-//     and the compile-time variant agrees with the run-time one.
+//     and the compile-time variant agrees with the run-time one;
+//   * row_list_size holds the items of any distribution of records over rows.
 // Prints "host logic ok <checks>" and exits 0, or the first failure and 1.
+#include <algorithm>
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
@@ -105,6 +107,25 @@ int main() {
     const int o = offset_octant(v[q & 1], v[(q >> 1) & 1], v[(q >> 2) & 1], 3);
     if (o != q) FAIL("octant %d -> %d", q, o);
     if (offset_octant(v[q & 1], v[(q >> 1) & 1], v[(q >> 2) & 1], 2) != (q & 3)) FAIL("quadrant %d", q);
+    ++checks;
+  }
+  // dense rows: evenly filled, all in one row, rows just above the cap
+  for (int rep = 0; rep < 3000; ++rep) {
+    TileGeo t{};
+    t.nq = rep & 1 ? 8 : 4;
+    const int nrows = 1 + (int)(rnd() % 5000);
+    t.nkeys = nrows * t.nq;
+    const long long np = (long long)(rnd() % (1ull << (rnd() % 31)));
+    const int cap = row_cap(np, t);
+    if (cap < 512 || cap % 128 || cap < np / 16384 || cap < 4 * np / nrows) FAIL("row_cap %d of %lld in %d", cap, np, nrows);
+    const int kind = rep % 3;
+    long long left = np, items = 0;
+    for (int r = 0; r < nrows && left > 0; ++r) {
+      long long c = kind == 0 ? np / nrows : kind == 1 ? left : std::min<long long>(left, cap + 1 + rnd() % 3);
+      left -= c;
+      if (c > cap) items += (c - cap + ROW_ITEM - 1) / ROW_ITEM;
+    }
+    if (items > row_list_size(np)) FAIL("%lld items of %lld records, list of %d", items, np, row_list_size(np));
     ++checks;
   }
   std::printf("host logic ok %lld\n", checks);
